@@ -1,17 +1,19 @@
 // Warp-cooperative group tree walk (the force hot path).
 //
 // One warp owns a group of at most 32 consecutive Morton-sorted targets (a run of sibling
-// subtrees cut from the octree, bz_groups.cu).  It walks the tree once for the whole group: each step pops up to 32 nodes (one per lane), tests them against the
+// subtrees cut from the octree, bz_groups.cu).  It walks the tree once for the whole group: each
+// step takes the children of the four nodes opened last (one per lane), tests them against the
 // group's bounding box, and sorts them with warp votes into
 //   - pruned (beyond the short-range cutoff),
 //   - accepted multipoles  -> appended to a shared-memory node list,
 //   - leaves to sum directly -> appended to a shared-memory leaf list,
-//   - opened internal nodes -> children pushed on a shared-memory stack (shuffle scan).
-// Full lists are flushed: every lane evaluates its own target against each listed node, and
-// leaf particles are pulled into a shared-memory tile with cp.async.bulk (global -> shared,
-// completing on an mbarrier, into this CTA only) and summed with FP32 pair arithmetic.
-// Per-flush partial sums are folded into the running force with a two-sum (compensated
-// accumulation).
+//   - opened internal nodes -> pushed on a shared-memory stack as (first child, child count),
+//     placed by a vote (pushing the children themselves took a shuffle scan and a loop).
+// Full lists are flushed: the lanes share the evaluation of every target against each listed
+// node (LaneMap), and leaf particles are pulled into a shared-memory tile with cp.async.bulk
+// (global -> shared, completing on an mbarrier, into this CTA only) and summed with FP32 pair
+// arithmetic.  Per-flush partial sums are folded into the running force with a two-sum
+// (compensated accumulation).
 //
 // Decisions are computed with round-to-nearest intrinsics (no contraction) so that the set
 // of accepted nodes and direct leaves is bit-identical to the oracle's; the reference's
@@ -26,9 +28,10 @@ namespace bz {
 namespace {
 
 constexpr int kWarps = 4;
-constexpr int kStack = 512;       // shared-memory part of the traversal stack
+constexpr int kStack = 128;       // shared-memory part of the traversal stack
 constexpr int kSpill = 8192;      // per-warp global spill area (oldest entries)
-constexpr int kList = 64;
+constexpr int kList = 64;         // leaf list
+constexpr int kNodes = 128;       // accepted nodes evaluated per flush
 constexpr int kTile = 128;
 constexpr int kFlushParticles = 256;  // listed leaf particles that trigger a flush
 constexpr int kIndexBits = 26;
@@ -37,26 +40,67 @@ constexpr int kPerPairImage = 64;  // leaf code: periodic image chosen per pair
 
 constexpr int kNoShift = 21;       // shift code of the central image on all three axes
 
-struct __align__(16) WarpSmem {
-    float4 tile[kTile];
+template <bool QUAD> struct __align__(16) WarpSmem {
+    // a leaf flush and a node flush never overlap: they share their staging area
     union {
         struct {
-            float4 nd_mono[32];
-            float4 nd_qa[32];
+            float4 tile[kTile];
+            unsigned mask[kTile / 32][32];  // per-lane in-cutoff bits of the tile
         };
-        unsigned mask[kTile / 32][32];  // leaf flush: per-lane in-cutoff bits of the tile
+        struct {
+            // accepted nodes, two to an entry so that packed FP32 instructions take both:
+            // {x x y y}, {z z m m}, {xx xx xy xy}, {xz xz yy yy}, {yz yz zz zz}
+            float4 nd[QUAD ? 5 : 2][kNodes / 2];
+            float2 nd_tr[QUAD ? kNodes / 2 : 1];  // tr(Q) eps^2 (Newtonian) or -tr(Q) / 2 (split)
+        };
     };
-    float2 nd_qb[32];
-    float nd_tr[32];  // -tr(Q) eps^2 / 3 of each node (traceless Newtonian form only)
-    int tidx[kTile];  // sorted index of each tile source (only when pairs are recorded)
-    int stack[kStack];
-    int nlist[kList];
+    float4 tgt[32];   // the group's targets (slots past its size repeat the first)
+    int tidx[kTile];  // sorted index of each tile source (pairs recorded, potentials)
+    unsigned stack[kStack];  // opened nodes: first child | (children - 1) << kIndexBits
+    int nlist[kNodes + 32];
     int lstart[kList];
     int lcount[kList];
     int lcode[kList];
     int lnode[kList];
     int lpre[kList];
     unsigned long long bar;
+};
+
+// How the 32 lanes share the evaluation of a group's gn targets against a staged list of
+// sources or nodes: lane = slice x T + slot with T target slots and S = 32 / T slices.  A lane
+// takes every S-th entry of the list for the targets slot, slot + T, ... (kChunk of them at a
+// time, so that one shared-memory read of an entry serves kChunk interactions), and the
+// slices' sums are combined once a flush.  With one target a lane instead, groups of fewer than
+// 32 targets leave lanes idle on every entry, and groups cut from an octree hold 18 (Plummer
+// 65k) to 23 (Hernquist 4M) of 32 on average, mostly a single particle in the outskirts of a
+// small system (1272 of the 1423 groups of Plummer 4096).  T = 4 rounds gn up to a multiple of 4.
+//
+// The kernel is bound by the issue and the FP32 pipe (Hernquist 1M: DRAM idle, FMA pipes 60 %
+// busy).  Measured per walk, one target a lane -> this mapping with two nodes or sources in
+// each packed FP32 instruction, 128 nodes a flush, and opened nodes instead of children on the
+// stack: Plummer 4096 0.233 -> 0.103 ms, Plummer 65k 0.64 -> 0.39 ms, Hernquist 4M 49.7 -> 36.4
+// ms, an adaptive ensemble substep of 96 clusters 1.12 -> 0.58 ms on average, isolated TreePM of
+// 1M (with the leaves wholly inside the cutoff summed without the filter) 6.87 -> 4.37 ms.  Four targets a
+// chunk (more code than the instruction cache holds: 42.6 ms at 4M) and scalar instructions
+// (40.0 ms) were slower.
+constexpr int kSlots = 4;
+constexpr int kChunk = 2;
+
+struct LaneMap {
+    int slot, slice, nslices, rows;  // rows: targets a slot serves
+    __device__ LaneMap(int gn, bool sliced)
+    {
+        const int lane = threadIdx.x & 31;
+        // log2 of the slots: 1 or 2 targets take as many, more take kSlots; a (nearly) full group
+        // has no lanes to win and takes one target a lane, which needs no sums over slices
+        // (all-full lattice groups, 128^3 CIC TreePM: 2.26 ms against 2.84; Hernquist 4M 36.4
+        // against 36.7)
+        const int sh = !sliced || gn > 28 ? 5 : (gn < 3 ? gn - 1 : 2);
+        slot = lane & ((1 << sh) - 1);
+        slice = lane >> sh;
+        nslices = 32 >> sh;
+        rows = sh == 2 ? (gn + kSlots - 1) / kSlots : 1;
+    }
 };
 
 // erfc(u) ~= t (a1 + t (a2 + t (a3 + t (a4 + t a5)))) e^{-u^2},  t = 1/(1 + p u)
@@ -89,6 +133,45 @@ __device__ __forceinline__ float ex2_approx(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+
+// Two FP32 values in one 64-bit register pair: one packed instruction does both.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ F2 f2(float a) { return f2(a, a); }
+__device__ __forceinline__ float lo(F2 a)
+{
+    return __uint_as_float(static_cast<unsigned>(a.v));
+}
+__device__ __forceinline__ float hi(F2 a)
+{
+    return __uint_as_float(static_cast<unsigned>(a.v >> 32));
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 rsqrt2(F2 a) { return f2(rsqrt_approx(lo(a)), rsqrt_approx(hi(a))); }
 
 template <bool SPLIT, bool POT>
 __device__ __forceinline__ void pair_pp(const float4 s, float tx, float ty, float tz,
@@ -222,31 +305,96 @@ __device__ __forceinline__ void pair_pn(const float4 mo, const float4 qa, const 
     }
 }
 
-// Force-only Newtonian quadrupole interaction with the traceless second moment
-// Q' = Q - tr(Q)/3 I.  With softening the trace does not drop out of the expansion; written with
-// Q' the acceleration is (m/s^3 + 15/2 (dQ'd + trm)/s^7) d - 3 Q'd/s^5 with s^2 = r^2 + eps^2 and
-// trm = -tr(Q) eps^2/3, algebraically the same as the traceful form (the m/s^3 + (15/2 dQd/s^7 -
+// Force-only Newtonian quadrupole interaction of two nodes at a time, with the traceless second
+// moment Q' = Q - tr(Q)/3 I.  With softening the trace does not drop out of the expansion; written
+// with Q' the acceleration is (m/s^3 + 15/2 (dQ'd + trm)/s^7) d - 3 Q'd/s^5 with s^2 = r^2 + eps^2
+// and trm = -tr(Q) eps^2/3, algebraically the same as the traceful form (the m/s^3 + (15/2 dQd/s^7 -
 // 3/2 tr/s^5)) d - 3 Qd/s^5 of pair_pn).  Used only when eps^2 exceeds the minimum distance^2,
 // so the minimum-distance guard of pair_pn can never trigger.
-__device__ __forceinline__ void pair_pn_newton(const float4 mo, const float4 qa, const float2 qb,
-                                               float trm, float tx, float ty, float tz, float eps2,
-                                               float& fx, float& fy, float& fz)
+// nx, ny, nz: the target's negated position; q = -3 Q' (xx xy xz yy yz zz), trm scaled by -3 too.
+__device__ __forceinline__ void pair_pn_newton2(F2 x, F2 y, F2 z, F2 m, const F2* q, F2 trm, F2 nx,
+                                                F2 ny, F2 nz, F2 eps2, F2& fx, F2& fy, F2& fz)
 {
-    const float dx = mo.x - tx, dy = mo.y - ty, dz = mo.z - tz;
-    const float s2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-    const float rinv = rsqrt_approx(s2);
-    const float a = rinv * rinv;       // 1/r^2
-    const float b = rinv * a;          // 1/r^3
-    const float t5 = b * a;            // 1/r^5
-    const float qdx = fmaf(qa.x, dx, fmaf(qa.y, dy, qa.z * dz));
-    const float qdy = fmaf(qa.y, dx, fmaf(qa.w, dy, qb.x * dz));
-    const float qdz = fmaf(qa.z, dx, fmaf(qb.x, dy, qb.y * dz));
-    const float dqd = fmaf(dx, qdx, fmaf(dy, qdy, fmaf(dz, qdz, trm)));
-    const float c0 = fmaf(7.5f * t5, a * dqd, mo.w * b);
-    const float n2 = -3.0f * t5;
-    fx = fmaf(c0, dx, fmaf(n2, qdx, fx));
-    fy = fmaf(c0, dy, fmaf(n2, qdy, fy));
-    fz = fmaf(c0, dz, fmaf(n2, qdz, fz));
+    const F2 dx = add2(x, nx), dy = add2(y, ny), dz = add2(z, nz);
+    const F2 rinv = rsqrt2(fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, eps2))));
+    const F2 a = mul2(rinv, rinv);  // 1/r^2
+    const F2 b = mul2(rinv, a);     // 1/r^3
+    const F2 t5 = mul2(b, a);       // 1/r^5
+    const F2 qx = fma2(q[0], dx, fma2(q[1], dy, mul2(q[2], dz)));
+    const F2 qy = fma2(q[1], dx, fma2(q[3], dy, mul2(q[4], dz)));
+    const F2 qz = fma2(q[2], dx, fma2(q[4], dy, mul2(q[5], dz)));
+    const F2 dqd = fma2(dx, qx, fma2(dy, qy, fma2(dz, qz, trm)));
+    const F2 c0 = mul2(b, fma2(mul2(a, mul2(a, dqd)), f2(-2.5f), m));
+    fx = fma2(c0, dx, fma2(t5, qx, fx));
+    fy = fma2(c0, dy, fma2(t5, qy, fy));
+    fz = fma2(c0, dz, fma2(t5, qz, fz));
+}
+
+// Force-only quadrupole interaction with the split kernel of two nodes at a time, softening above
+// the minimum-distance floor.  pair_pn's expansion with its powers of 1/s factored out:
+//   f = b (m h + a (l a dQd / 2 - k tr / 2)) d - k a b Q d,   a = 1/s^2, b = 1/s^3.
+// nx, ny, nz: the target's negated position; q = -Q (xx xy xz yy yz zz), htr = -tr(Q) / 2.
+__device__ __forceinline__ void pair_pn_split2(F2 x, F2 y, F2 z, F2 m, const F2* q, F2 htr, F2 nx, F2 ny,
+                                               F2 nz, F2 eps2, float inv2rs, F2& fx, F2& fy, F2& fz)
+{
+    const F2 dx = add2(x, nx), dy = add2(y, ny), dz = add2(z, nz);
+    const F2 s2 = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, eps2)));
+    const F2 rinv = rsqrt2(s2);
+    const F2 a = mul2(rinv, rinv);
+    const F2 b = mul2(rinv, a);
+    const F2 u = mul2(mul2(s2, rinv), f2(inv2rs));
+    const F2 u2 = mul2(u, u);
+    const F2 g = mul2(u2, f2(-1.4426950408889634f));
+    const F2 e = f2(ex2_approx(lo(g)), ex2_approx(hi(g)));
+    const F2 v = fma2(u, f2(0.3275911f), f2(1.0f));
+    const F2 t = f2(rcp_approx(lo(v)), rcp_approx(hi(v)));
+    F2 ec = f2(1.061405429f);
+    ec = fma2(ec, t, f2(-1.453152027f));
+    ec = fma2(ec, t, f2(1.421413741f));
+    ec = fma2(ec, t, f2(-0.284496736f));
+    ec = fma2(ec, t, f2(0.254829592f));
+    ec = mul2(mul2(ec, t), e);
+    const F2 w1 = mul2(u, e), w3 = mul2(u2, w1), w5 = mul2(u2, w3);
+    const F2 h = fma2(w1, f2(kTwoOverSqrtPi), ec);
+    const F2 k = fma2(w3, f2(kFourOverSqrtPi), mul2(h, f2(3.0f)));
+    const F2 nl = fma2(w5, f2(-0.5f * kEightOverSqrtPi), mul2(k, f2(-2.5f)));  // -l / 2
+    const F2 qx = fma2(q[0], dx, fma2(q[1], dy, mul2(q[2], dz)));
+    const F2 qy = fma2(q[1], dx, fma2(q[3], dy, mul2(q[4], dz)));
+    const F2 qz = fma2(q[2], dx, fma2(q[4], dy, mul2(q[5], dz)));
+    const F2 dqd = fma2(dx, qx, fma2(dy, qy, mul2(dz, qz)));
+    const F2 c0 = mul2(b, fma2(a, fma2(mul2(nl, a), dqd, mul2(k, htr)), mul2(m, h)));
+    const F2 c2 = mul2(k, mul2(a, b));
+    fx = fma2(c0, dx, fma2(c2, qx, fx));
+    fy = fma2(c0, dy, fma2(c2, qy, fy));
+    fz = fma2(c0, dz, fma2(c2, qz, fz));
+}
+
+// As pair_fast without a cutoff, for two sources at a time.
+template <bool SPLIT>
+__device__ __forceinline__ void pair_fast2(F2 x, F2 y, F2 z, F2 m, F2 nx, F2 ny, F2 nz, F2 eps2,
+                                           const SplitK& k, F2& fx, F2& fy, F2& fz)
+{
+    const F2 dx = add2(x, nx), dy = add2(y, ny), dz = add2(z, nz);
+    const F2 s2 = add2(fma2(dx, dx, fma2(dy, dy, mul2(dz, dz))), eps2);
+    const F2 rinv = rsqrt2(s2);
+    F2 mw = m;
+    if (SPLIT) {
+        const F2 sd = mul2(s2, rinv);
+        const F2 g = mul2(s2, f2(k.cexp));
+        const F2 e = f2(ex2_approx(lo(g)), ex2_approx(hi(g)));
+        const F2 u = fma2(sd, f2(k.pk), f2(1.0f));
+        const F2 t = f2(rcp_approx(lo(u)), rcp_approx(hi(u)));
+        F2 q = f2(1.061405429f);
+        q = fma2(q, t, f2(-1.453152027f));
+        q = fma2(q, t, f2(1.421413741f));
+        q = fma2(q, t, f2(-0.284496736f));
+        q = fma2(q, t, f2(0.254829592f));
+        mw = mul2(m, mul2(e, fma2(t, q, mul2(sd, f2(k.c2)))));
+    }
+    const F2 f = mul2(mw, mul2(rinv, mul2(rinv, rinv)));
+    fx = fma2(f, dx, fx);
+    fy = fma2(f, dy, fy);
+    fz = fma2(f, dz, fz);
 }
 
 struct Acc {
@@ -267,23 +415,96 @@ struct Acc {
     __device__ float total(int i) const { return s[i] + e[i]; }
 };
 
+template <int N> struct IntC {
+    static constexpr int value = N;
+};
+
 __device__ __forceinline__ float shift_of(int code, int axis, float box)
 {
     return box * static_cast<float>(((code >> (2 * axis)) & 3) - 1);
 }
 
+// Sums of one pass over a staged list: R targets of this lane's slot, C components.
+template <int R, int C> struct Rows {
+    float tx[R], ty[R], tz[R], f[C][R];
+    template <class W> __device__ __forceinline__ void load(const W& w, const LaneMap& lm, int row0)
+    {
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const float4 t = w.tgt[lm.slot + kSlots * (row0 + k)];
+            tx[k] = t.x;
+            ty[k] = t.y;
+            tz[k] = t.z;
+#pragma unroll
+            for (int c = 0; c < C; ++c)
+                f[c][k] = 0.0f;
+        }
+    }
+    // Adds the slices' sums; lane j = slice * slots + slot adds those of target j to acc.  (Two
+    // rows only go with kSlots slots, a single one with any number.)
+    __device__ __forceinline__ void fold(const LaneMap& lm, int row0, Acc& acc)
+    {
+        if constexpr (R == 2) {
+            // the first exchange leaves a lane with the row of its slice's parity
+            const bool odd = lm.slice & 1;
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                float v = (odd ? f[c][1] : f[c][0]) +
+                          __shfl_xor_sync(kFullMask, odd ? f[c][0] : f[c][1], kSlots);
+                v += __shfl_xor_sync(kFullMask, v, 2 * kSlots);
+                v += __shfl_xor_sync(kFullMask, v, 4 * kSlots);
+                acc.add(c, (lm.slice & ~1) == row0 ? v : 0.0f);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                float v = f[c][0];
+                for (int o = 16; o >= 32 / lm.nslices; o >>= 1)
+                    v += __shfl_xor_sync(kFullMask, v, o);
+                acc.add(c, lm.slice == row0 ? v : 0.0f);
+            }
+        }
+    }
+};
+
+// The walks that slice: all but the short-range walk without quadrupoles (a node-size cap or
+// multipole_order 1), which the per-lane cutoff filter dominates: its few node terms do not pay
+// for the registers of the chunks.
+template <bool SPLIT, bool QUAD> constexpr bool walk_sliced() { return !SPLIT || QUAD; }
+
+// Calls body with every chunk of at most kChunk rows: body(std::integral_constant<R>, row0).
+template <bool SLICED, class F> __device__ __forceinline__ void for_rows(const LaneMap& lm, F body)
+{
+    if constexpr (!SLICED) {
+        body(IntC<1>{}, 0);
+    } else
+    for (int row0 = 0; row0 < lm.rows; row0 += kChunk) {
+        if (lm.rows - row0 >= kChunk)
+            body(IntC<kChunk>{}, row0);
+        else
+            body(IntC<1>{}, row0);
+    }
+}
+
+// Evaluates the first m <= kNodes listed nodes for the group's targets.
 template <bool PERIODIC, bool SPLIT, bool QUAD, bool POT>
-__device__ __forceinline__ void flush_nodes(WarpSmem& w, int nn, const TreeArrays& t,
-                                            const WalkParams& p, float inv2rs, float tx,
-                                            float ty, float tz, Acc& acc)
+__device__ __forceinline__ void flush_nodes(WarpSmem<QUAD>& w, int m, const TreeArrays& t,
+                                            const WalkParams& p, float inv2rs, const LaneMap& lm,
+                                            Acc& acc)
 {
     const int lane = threadIdx.x & 31;
-    // Newtonian force-only quadrupoles take the traceless form; it needs eps^2 > min distance^2
-    const bool newton = !SPLIT && QUAD && !POT && p.eps2 > p.min_dist2;
-    for (int base = 0; base < nn; base += 32) {
-        const int m = min(32, nn - base);
-        if (lane < m) {
-            const int e = w.nlist[base + lane];
+    // force-only quadrupoles with eps^2 > min distance^2 are evaluated two nodes at a time; the
+    // Newtonian ones in the traceless form
+    const bool packed = QUAD && !POT && p.eps2 > p.min_dist2;
+    const int pairs = (m + 1) >> 1;
+    if ((m & 1) && lane == 0)
+        w.nlist[m] = w.nlist[m - 1];  // an odd list's last node is paired with itself, massless
+    __syncwarp();
+    for (int i = lane; i < pairs; i += 32) {
+        float v[2][11];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int e = w.nlist[2 * i + h];
             const int k = e & kIndexMask;
             float4 mo = t.mono[k];
             if (PERIODIC) {
@@ -292,58 +513,115 @@ __device__ __forceinline__ void flush_nodes(WarpSmem& w, int nn, const TreeArray
                 mo.y -= shift_of(code, 1, p.box);
                 mo.z -= shift_of(code, 2, p.box);
             }
-            w.nd_mono[lane] = mo;
+            v[h][0] = mo.x;
+            v[h][1] = mo.y;
+            v[h][2] = mo.z;
+            v[h][3] = mo.w;
             if (QUAD) {
-                float4 qa = t.quadA[k];
-                float2 qb = t.quadB[k];
-                if (newton) {
+                const float4 qa = t.quadA[k];
+                const float2 qb = t.quadB[k];
+                v[h][4] = qa.x;
+                v[h][5] = qa.y;
+                v[h][6] = qa.z;
+                v[h][7] = qa.w;
+                v[h][8] = qb.x;
+                v[h][9] = qb.y;
+                if (packed) {
                     const float tr = qa.x + qa.w + qb.y;
-                    const float tr3 = tr * (1.0f / 3.0f);
-                    qa.x -= tr3;
-                    qa.w -= tr3;
-                    qb.y -= tr3;
-                    w.nd_tr[lane] = -tr3 * p.eps2;
+                    const float c = SPLIT ? -1.0f : -3.0f, off = SPLIT ? 0.0f : tr;
+                    v[h][4] = fmaf(c, qa.x, off);
+                    v[h][5] = c * qa.y;
+                    v[h][6] = c * qa.z;
+                    v[h][7] = fmaf(c, qa.w, off);
+                    v[h][8] = c * qb.x;
+                    v[h][9] = fmaf(c, qb.y, off);
+                    v[h][10] = SPLIT ? -0.5f * tr : tr * p.eps2;
                 }
-                w.nd_qa[lane] = qa;
-                w.nd_qb[lane] = qb;
             }
         }
-        __syncwarp();
-        float fx = 0.0f, fy = 0.0f, fz = 0.0f, fp = 0.0f;
-        if (newton) {
-            int j = 0;
-            for (; j + 1 < m; j += 2) {
-                pair_pn_newton(w.nd_mono[j], w.nd_qa[j], w.nd_qb[j], w.nd_tr[j], tx, ty, tz, p.eps2,
-                               fx, fy, fz);
-                pair_pn_newton(w.nd_mono[j + 1], w.nd_qa[j + 1], w.nd_qb[j + 1], w.nd_tr[j + 1], tx,
-                               ty, tz, p.eps2, fx, fy, fz);
-            }
-            if (j < m)
-                pair_pn_newton(w.nd_mono[j], w.nd_qa[j], w.nd_qb[j], w.nd_tr[j], tx, ty, tz, p.eps2,
-                               fx, fy, fz);
-        } else {
-            for (int j = 0; j < m; ++j) {
-                const float4 qa = QUAD ? w.nd_qa[j] : make_float4(0, 0, 0, 0);
-                const float2 qb = QUAD ? w.nd_qb[j] : make_float2(0, 0);
-                pair_pn<SPLIT, QUAD, POT>(w.nd_mono[j], qa, qb, tx, ty, tz, p, inv2rs, fx, fy, fz, fp);
-            }
+        if (2 * i + 1 == m) {
+#pragma unroll
+            for (int c = 3; c < 11; ++c)
+                v[1][c] = 0.0f;
         }
-        acc.add(0, fx);
-        acc.add(1, fy);
-        acc.add(2, fz);
-        if (POT)
-            acc.add(3, fp);
-        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < (QUAD ? 5 : 2); ++c)
+            w.nd[c][i] = make_float4(v[0][2 * c], v[1][2 * c], v[0][2 * c + 1], v[1][2 * c + 1]);
+        if (packed)
+            w.nd_tr[i] = make_float2(v[0][10], v[1][10]);
     }
+    __syncwarp();
+    for_rows<walk_sliced<SPLIT, QUAD>()>(lm, [&](auto rc, int row0) {
+        constexpr int R = decltype(rc)::value;
+        Rows<R, POT ? 4 : 3> rows;
+        rows.load(w, lm, row0);
+        float none = 0.0f;
+        if (packed) {
+            F2 nx[R], ny[R], nz[R], fx[R], fy[R], fz[R];
+            const F2 eps2 = f2(p.eps2);
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                nx[k] = f2(-rows.tx[k]);
+                ny[k] = f2(-rows.ty[k]);
+                nz[k] = f2(-rows.tz[k]);
+                fx[k] = fy[k] = fz[k] = f2(0.0f);
+            }
+#pragma unroll 1
+            for (int j = lm.slice; j < pairs; j += lm.nslices) {
+                const ulonglong2* nd = reinterpret_cast<const ulonglong2*>(&w.nd[0][j]);
+                constexpr int st = QUAD ? kNodes / 2 : 0;  // (packed implies QUAD)
+                const ulonglong2 a = nd[0], b = nd[st], c = nd[2 * st], d = nd[3 * st], e = nd[4 * st];
+                const F2 tr{*reinterpret_cast<const unsigned long long*>(&w.nd_tr[QUAD ? j : 0])};
+                const F2 q[6] = {{c.x}, {c.y}, {d.x}, {d.y}, {e.x}, {e.y}};
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    if (SPLIT)
+                        pair_pn_split2({a.x}, {a.y}, {b.x}, {b.y}, q, tr, nx[k], ny[k], nz[k], eps2, inv2rs,
+                                       fx[k], fy[k], fz[k]);
+                    else
+                        pair_pn_newton2({a.x}, {a.y}, {b.x}, {b.y}, q, tr, nx[k], ny[k], nz[k], eps2, fx[k],
+                                        fy[k], fz[k]);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                rows.f[0][k] = lo(fx[k]) + hi(fx[k]);
+                rows.f[1][k] = lo(fy[k]) + hi(fy[k]);
+                rows.f[2][k] = lo(fz[k]) + hi(fz[k]);
+            }
+        } else {
+#pragma unroll 1
+            for (int j = lm.slice; j < pairs; j += lm.nslices) {
+                const float4 a = w.nd[0][j], b = w.nd[1][j];
+                const float4 c = QUAD ? w.nd[QUAD ? 2 : 0][j] : make_float4(0, 0, 0, 0);
+                const float4 d = QUAD ? w.nd[QUAD ? 3 : 0][j] : make_float4(0, 0, 0, 0);
+                const float4 e = QUAD ? w.nd[QUAD ? 4 : 0][j] : make_float4(0, 0, 0, 0);
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    pair_pn<SPLIT, QUAD, POT>(make_float4(a.x, a.z, b.x, b.z), make_float4(c.x, c.z, d.x, d.z),
+                                              make_float2(e.x, e.z), rows.tx[k], rows.ty[k], rows.tz[k], p,
+                                              inv2rs, rows.f[0][k], rows.f[1][k], rows.f[2][k],
+                                              POT ? rows.f[POT ? 3 : 0][k] : none);
+                    pair_pn<SPLIT, QUAD, POT>(make_float4(a.y, a.w, b.y, b.w), make_float4(c.y, c.w, d.y, d.w),
+                                              make_float2(e.y, e.w), rows.tx[k], rows.ty[k], rows.tz[k], p,
+                                              inv2rs, rows.f[0][k], rows.f[1][k], rows.f[2][k],
+                                              POT ? rows.f[POT ? 3 : 0][k] : none);
+                }
+            }
+        }
+        __syncwarp();
+        rows.fold(lm, row0, acc);
+    });
+    __syncwarp();
 }
 
-template <bool PERIODIC, bool SPLIT, bool POT>
-__device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* __restrict__ pos4,
+template <bool PERIODIC, bool SPLIT, bool POT, bool SLICED, class W>
+__device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure, const float4* __restrict__ pos4,
                                              const TreeArrays& t, const WalkParams& p,
                                              float inv2rs, bool cut, float tx, float ty, float tz,
                                              int self_index, Acc& acc, uint32_t& phase, int* err,
                                              const WalkOutputs& o, int pair_row, int& npair,
-                                             unsigned& evald)
+                                             unsigned& evald, const LaneMap& lm)
 {
     // pairs closer than rcorr are recorded for the learned correction (pair_row < 0: a lane
     // without a target records nothing)
@@ -359,6 +637,7 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
     const int lane = threadIdx.x & 31;
     // Force-only evaluation above the minimum-distance floor runs the per-lane cutoff filter
     const bool fast = !POT && p.eps2 > p.min_dist2;
+    cut = cut && !sure;  // every pair of these leaves lies inside the cutoff
     if (cut && !fast) {
         // Drop leaves that no target of this warp can reach: a leaf whose (shifted) box is
         // farther than the cutoff from every lane's target holds no pair inside the cutoff.
@@ -375,9 +654,9 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
             hi[h] = lo[h];
             ppi[h] = false;
             if (j < nl) {
-                const int code = w.lcode[j];
+                const int code = w.lcode[first + j];
                 ppi[h] = PERIODIC && code == kPerPairImage;
-                const int k = w.lnode[j];
+                const int k = w.lnode[first + j];
                 const float4 b0 = t.box0[k];
                 const float4 b1 = t.box1[k];
                 float sxo = 0.0f, syo = 0.0f, szo = 0.0f;
@@ -410,10 +689,10 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
             }
             if (__any_sync(kFullMask, need)) {
                 if (lane == 0 && keep != j) {
-                    w.lstart[keep] = w.lstart[j];
-                    w.lcount[keep] = w.lcount[j];
-                    w.lcode[keep] = w.lcode[j];
-                    w.lnode[keep] = w.lnode[j];
+                    w.lstart[first + keep] = w.lstart[first + j];
+                    w.lcount[first + keep] = w.lcount[first + j];
+                    w.lcode[first + keep] = w.lcode[first + j];
+                    w.lnode[first + keep] = w.lnode[first + j];
                 }
                 ++keep;
             }
@@ -424,16 +703,16 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
             return;
     }
     // exclusive prefix of the leaf sizes (list holds at most 64 entries)
-    const int c0 = lane < nl ? w.lcount[lane] : 0;
-    const int c1 = lane + 32 < nl ? w.lcount[lane + 32] : 0;
+    const int c0 = lane < nl ? w.lcount[first + lane] : 0;
+    const int c1 = lane + 32 < nl ? w.lcount[first + lane + 32] : 0;
     const int i0 = warp_incl_scan(c0);
     const int t0 = __shfl_sync(kFullMask, i0, 31);
     const int i1 = warp_incl_scan(c1) + t0;
     const int total = __shfl_sync(kFullMask, i1, 31);
     if (lane < nl)
-        w.lpre[lane] = i0 - c0;
+        w.lpre[first + lane] = i0 - c0;
     if (lane + 32 < nl)
-        w.lpre[lane + 32] = i1 - c1;
+        w.lpre[first + lane + 32] = i1 - c1;
     __syncwarp();
     SplitK sk;
     sk.inv2rs = inv2rs;
@@ -453,24 +732,24 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
         // image shift or per-pair images
         bool shifted = false, pairimg = false;
         for (int j = lane; j < nl; j += 32) {
-            const int lo = max(w.lpre[j], cbase);
-            const int hi = min(w.lpre[j] + w.lcount[j], cend);
+            const int lo = max(w.lpre[first + j], cbase);
+            const int hi = min(w.lpre[first + j] + w.lcount[first + j], cend);
             if (hi > lo) {
-                bulk_g2s(&w.tile[lo - cbase], pos4 + (w.lstart[j] + (lo - w.lpre[j])),
+                bulk_g2s(&w.tile[lo - cbase], pos4 + (w.lstart[first + j] + (lo - w.lpre[first + j])),
                          static_cast<uint32_t>(hi - lo) * 16u, &w.bar);
                 if (PERIODIC) {
-                    const int code = w.lcode[j];
+                    const int code = w.lcode[first + j];
                     pairimg = pairimg || code == kPerPairImage;
                     shifted = shifted || (code != kNoShift && code != kPerPairImage);
                 }
-                if (rec)
+                if (rec || POT)
                     for (int q = lo; q < hi; ++q)
-                        w.tidx[q - cbase] = w.lstart[j] + (q - w.lpre[j]);
+                        w.tidx[q - cbase] = w.lstart[first + j] + (q - w.lpre[first + j]);
             }
         }
         const bool any_shift = PERIODIC && __any_sync(kFullMask, shifted);
         const bool per_pair = PERIODIC && __any_sync(kFullMask, pairimg);
-        if (rec)
+        if (rec || POT)
             __syncwarp();
         mbar_wait_bounded(&w.bar, phase, err);
         phase ^= 1u;
@@ -479,9 +758,9 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
         // positions).  Tiles without shifted leaves, most of them, skip this.
         if (any_shift) {
             for (int j = lane; j < nl; j += 32) {
-                const int lo = max(w.lpre[j], cbase);
-                const int hi = min(w.lpre[j] + w.lcount[j], cend);
-                const int code = w.lcode[j];
+                const int lo = max(w.lpre[first + j], cbase);
+                const int hi = min(w.lpre[first + j] + w.lcount[first + j], cend);
+                const int code = w.lcode[first + j];
                 if (hi <= lo || code == kNoShift || code == kPerPairImage)
                     continue;
                 const float shx = shift_of(code, 0, p.box), shy = shift_of(code, 1, p.box),
@@ -495,13 +774,71 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
             }
             __syncwarp();
         }
+        const int nb = cend - cbase;
+        if (!per_pair && !rec && !(fast && cut)) {
+            // every listed source of the tile goes through the pair law, two at a time (the tile
+            // filled up with massless sources to whole pairs for every slice)
+            evald += nb;
+            const int npad = (nb + 2 * lm.nslices - 1) & ~(2 * lm.nslices - 1);
+            if (SLICED && fast) {
+                for (int j = nb + lane; j < npad; j += 32)
+                    w.tile[j] = make_float4(tx, ty, tz, 0.0f);
+                __syncwarp();
+            }
+            for_rows<SLICED>(lm, [&](auto rc, int row0) {
+                constexpr int R = decltype(rc)::value;
+                Rows<R, POT ? 4 : 3> rows;
+                rows.load(w, lm, row0);
+                float none = 0.0f;
+                if (SLICED && fast) {
+                    F2 nx[R], ny[R], nz[R], fx[R], fy[R], fz[R];
+                    const F2 eps2 = f2(p.eps2);
+#pragma unroll
+                    for (int k = 0; k < R; ++k) {
+                        nx[k] = f2(-rows.tx[k]);
+                        ny[k] = f2(-rows.ty[k]);
+                        nz[k] = f2(-rows.tz[k]);
+                        fx[k] = fy[k] = fz[k] = f2(0.0f);
+                    }
+#pragma unroll 1
+                    for (int j = lm.slice; j < npad; j += 2 * lm.nslices) {
+                        const float4 s0 = w.tile[j], s1 = w.tile[j + lm.nslices];
+                        const F2 x = f2(s0.x, s1.x), y = f2(s0.y, s1.y), z = f2(s0.z, s1.z), m = f2(s0.w, s1.w);
+#pragma unroll
+                        for (int k = 0; k < R; ++k)
+                            pair_fast2<SPLIT>(x, y, z, m, nx[k], ny[k], nz[k], eps2, sk, fx[k], fy[k], fz[k]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < R; ++k) {
+                        rows.f[0][k] = lo(fx[k]) + hi(fx[k]);
+                        rows.f[1][k] = lo(fy[k]) + hi(fy[k]);
+                        rows.f[2][k] = lo(fz[k]) + hi(fz[k]);
+                    }
+                } else {
+                    const int t0 = self_index - lane + lm.slot + kSlots * row0;
+#pragma unroll 1
+                    for (int j = lm.slice; j < nb; j += lm.nslices) {
+                        const float4 s4 = w.tile[j];
+                        const int src = POT ? w.tidx[j] : 0;
+#pragma unroll
+                        for (int k = 0; k < R; ++k)
+                            pair_pp<SPLIT, POT>(s4, rows.tx[k], rows.ty[k], rows.tz[k], p, inv2rs, cut,
+                                                POT && src == t0 + kSlots * k, rows.f[0][k], rows.f[1][k],
+                                                rows.f[2][k], POT ? rows.f[POT ? 3 : 0][k] : none);
+                    }
+                }
+                __syncwarp();
+                rows.fold(lm, row0, acc);
+            });
+            __syncwarp();
+            continue;
+        }
         float fx = 0.0f, fy = 0.0f, fz = 0.0f, fp = 0.0f;
         if (fast && cut && !per_pair) {
             // Cutoff filter: each lane marks the tile sources inside its own cutoff sphere
             // (the same r^2 expression as the pair law, so the set is exact), then sums only
             // those.  Skipped pairs contribute exactly zero in the unfiltered sum, so the
             // result is bit-identical to summing every listed source in tile order.
-            const int nb = cend - cbase;
             const int nw = (nb + 31) >> 5;
             // r2 <= rcut2 exactly when r2 - next_float(rcut2) is negative (a float difference
             // has the exact sign), so the sign bit is the mask bit: one funnel shift appends it
@@ -549,18 +886,18 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
             // here: that path skips the leaves that end before its tile)
         } else {
             for (int j = jfirst; j < nl; ++j) {
-                const int pre = w.lpre[j];
+                const int pre = w.lpre[first + j];
                 if (pre >= cend)
                     break;
                 const int lo = max(pre, cbase);
-                const int hi = min(pre + w.lcount[j], cend);
+                const int hi = min(pre + w.lcount[first + j], cend);
                 if (hi <= lo)
                     continue;
-                const int gsrc0 = w.lstart[j] + (lo - pre);
+                const int gsrc0 = w.lstart[first + j] + (lo - pre);
                 const int off = lo - cbase;
                 const int cntp = hi - lo;
                 evald += cntp;  // every listed source goes through the pair law here
-                if (PERIODIC && w.lcode[j] == kPerPairImage) {
+                if (PERIODIC && w.lcode[first + j] == kPerPairImage) {
                     // rare slow path: nearest image chosen per pair
                     const float inv_box = 1.0f / p.box;
                     for (int q = 0; q < cntp; ++q) {
@@ -573,33 +910,22 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
                         if (rec)
                             record(s4, gsrc0 + q);
                     }
-                    if (pre + w.lcount[j] <= cend)
+                    if (pre + w.lcount[first + j] <= cend)
                         jfirst = j + 1;
                     continue;
                 }
-                int q = 0;
                 if (fast) {
-                    for (; q + 1 < cntp; q += 2) {
-                        pair_fast<SPLIT>(w.tile[off + q], tx, ty, tz, p.eps2, p.rcut2, cut, sk, fx, fy, fz);
-                        pair_fast<SPLIT>(w.tile[off + q + 1], tx, ty, tz, p.eps2, p.rcut2, cut, sk, fx, fy, fz);
-                    }
-                    if (q < cntp)
+                    for (int q = 0; q < cntp; ++q)
                         pair_fast<SPLIT>(w.tile[off + q], tx, ty, tz, p.eps2, p.rcut2, cut, sk, fx, fy, fz);
                 } else {
-                    for (; q + 1 < cntp; q += 2) {
-                        pair_pp<SPLIT, POT>(w.tile[off + q], tx, ty, tz, p, inv2rs, cut,
-                                            POT && gsrc0 + q == self_index, fx, fy, fz, fp);
-                        pair_pp<SPLIT, POT>(w.tile[off + q + 1], tx, ty, tz, p, inv2rs, cut,
-                                            POT && gsrc0 + q + 1 == self_index, fx, fy, fz, fp);
-                    }
-                    for (; q < cntp; ++q)
+                    for (int q = 0; q < cntp; ++q)
                         pair_pp<SPLIT, POT>(w.tile[off + q], tx, ty, tz, p, inv2rs, cut,
                                             POT && gsrc0 + q == self_index, fx, fy, fz, fp);
                 }
                 if (rec)
                     for (int q2 = 0; q2 < cntp; ++q2)
                         record(w.tile[off + q2], gsrc0 + q2);
-                if (pre + w.lcount[j] <= cend)
+                if (pre + w.lcount[first + j] <= cend)
                     jfirst = j + 1;
             }
         }
@@ -612,11 +938,20 @@ __device__ __forceinline__ void flush_leaves(WarpSmem& w, int nl, const float4* 
     }
 }
 
+// Resident blocks an SM that the walk is compiled for (4: 128 registers, 5: 96, 7: 72).  The
+// sliced evaluation keeps two nodes, two targets and their sums in packed registers: 4 blocks
+// hold them without spills (Hernquist 4M: 36.4 ms at 4, 37.4 at 5; isolated TreePM 1M: 4.35 at 4,
+// 4.45 at 5, 4.99 at 6).  The walk that only filters takes the warps.
+template <bool SPLIT, bool QUAD, bool POT> constexpr int walk_min_blocks()
+{
+    return SPLIT && !QUAD && !POT ? 7 : 4;
+}
+
 // Persistent kernel: each warp takes groups from a global queue until none are left.  The
 // traversal stack lives in shared memory; when it would overflow, its oldest half is spilled
 // to a per-warp-slot global area and refilled when the shared part runs dry.
 template <bool PERIODIC, bool SPLIT, bool QUAD, bool POT>
-__global__ void __launch_bounds__(kWarps * 32) k_walk(const float4* __restrict__ pos4, int n,
+__global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>()) k_walk(const float4* __restrict__ pos4, int n,
                                                        TreeArrays t, const int* __restrict__ gstart,
                                                        const int* __restrict__ groot,
                                                        const int* __restrict__ ngroups_ptr,
@@ -634,13 +969,14 @@ __global__ void __launch_bounds__(kWarps * 32) k_walk(const float4* __restrict__
     }
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    WarpSmem& w = reinterpret_cast<WarpSmem*>(smem_raw)[warp];
+    WarpSmem<QUAD>& w = reinterpret_cast<WarpSmem<QUAD>*>(smem_raw)[warp];
     int* spill = spill_base + static_cast<size_t>(blockIdx.x * kWarps + warp) * kSpill;
     const int ngroups = *ngroups_ptr;
     if (lane == 0)
         mbar_init(&w.bar, 1);
     fence_mbar_init();
     __syncwarp();
+    constexpr bool SLICED = walk_sliced<SPLIT, QUAD>();
     const bool cut = p.rcut2 > 0.0f;
     const float inv2rs = SPLIT ? 0.5f / p.rsplit : 0.0f;
     const float rcut = __fsqrt_rn(p.rcut2);
@@ -663,6 +999,8 @@ __global__ void __launch_bounds__(kWarps * 32) k_walk(const float4* __restrict__
         // adaptive steps: only groups holding a target that closes its step are walked
         if (p.active != nullptr && !__any_sync(kFullMask, valid && p.active[ti] != 0))
             continue;
+        const LaneMap lanes(gn, SLICED);
+        w.tgt[lane] = me;
         float gmin[3] = {me.x, me.y, me.z}, gmax[3] = {me.x, me.y, me.z};
 #pragma unroll
         for (int a = 0; a < 3; ++a)
@@ -677,171 +1015,206 @@ __global__ void __launch_bounds__(kWarps * 32) k_walk(const float4* __restrict__
             ghalf[a] = __fmul_rn(0.5f, __fsub_rn(gmax[a], gmin[a]));
         }
 
+        // With a cutoff, leaves wholly inside it for every target ("sure": the farthest corners of
+        // leaf and group) are listed from the far end of the leaf list and summed without the
+        // per-lane filter; the margin covers the rounding of a pair's own distance test.
+        const float sure2 = p.rcut2 * 0.9999f;
+        const bool sort_leaves = SLICED && cut && o.pair_src == nullptr &&
+                                 ghalf[0] * ghalf[0] + ghalf[1] * ghalf[1] + ghalf[2] * ghalf[2] < p.rcut2;
         if (lane == 0)
-            w.stack[0] = groot[g];  // the group's system root (node 0 for a single system)
+            w.stack[0] = static_cast<unsigned>(groot[g]);  // the group's system root, as one child
         __syncwarp();
-        int top = 1, gtop = 0, nn = 0, nl = 0, lp = 0;
-        unsigned long long cnt_pp = 0, cnt_pn = 0;
+        int top = 1, gtop = 0, nn = 0, nl = 0, ns = 0, lp = 0;
+        unsigned cnt_pp = 0, cnt_pn = 0;  // (a group lists a particle or a node at most once)
         Acc acc;
         acc.zero();
         int npair = 0;
         unsigned evald = 0;  // pairs this lane's target took through the pair law
-        bool bail = false;
-        while (top > 0 || gtop > 0) {
-            if (top == 0) {  // refill from the spill area (uniform branch)
-                const int m = min(gtop, kStack / 2);
-                for (int i = lane; i < m; i += 32)
-                    w.stack[i] = spill[gtop - m + i];
-                gtop -= m;
-                top = m;
+        // one traversal step (while nodes are left) and the flushes it makes due; the last turn
+        // flushes what is still listed
+        for (;;) {
+            const bool done = top == 0 && gtop == 0;
+            if (!done) {
+                if (top == 0) {  // refill from the spill area (uniform branch)
+                    const int m = min(gtop, kStack / 2);
+                    for (int i = lane; i < m; i += 32)
+                        w.stack[i] = static_cast<unsigned>(spill[gtop - m + i]);
+                    gtop -= m;
+                    top = m;
+                    __syncwarp();
+                }
+                // the children of the four nodes opened last, eight lanes a node
+                const int from = top - 1 - (lane >> 3);
+                const unsigned ent = w.stack[max(from, 0)];
+                const int child = lane & 7;
+                const bool on = from >= 0 && child <= static_cast<int>(ent >> kIndexBits);
+                const int k = on ? static_cast<int>(ent & kIndexMask) + child : -1;
+                top = max(top - 4, 0);
                 __syncwarp();
-            }
-            const int take = min(top, 32);
-            const int k = lane < take ? w.stack[top - take + lane] : -1;
-            top -= take;
-            __syncwarp();
-            bool accept = false, leaf = false;
-            int nch = 0, link = 0, info = 0, code = 0;
-            if (k >= 0) {
-                const float4 b0 = t.box0[k];
-                const float4 b1 = t.box1[k];
-                // the centre of mass matters only to a node that may be accepted; with a node
-                // size cap (TreePM) most nodes are too large, and skip the load
-                const bool capped = SPLIT && p.max_node_size > 0.0f;  // the cap is a TreePM setting
-                float4 mo = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (!capped)
-                    mo = t.mono[k];
-                link = __float_as_int(b0.w);
-                info = __float_as_int(b1.w);
-                const float bmin[3] = {b0.x, b0.y, b0.z}, bmax[3] = {b1.x, b1.y, b1.z};
-                float sh[3] = {0.0f, 0.0f, 0.0f};
-                bool amb = false;
-                if (PERIODIC) {
-                    // Image-ambiguous node (its extent + the group's + the cutoff reaches half
-                    // the box): always opened; a leaf is summed with per-pair minimum images.
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const float nh = __fmul_rn(0.5f, __fsub_rn(bmax[a], bmin[a]));
-                        if (__fadd_rn(__fadd_rn(ghalf[a], nh), rcut) > half_box)
-                            amb = true;
-                    }
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const float cn = __fmul_rn(0.5f, __fadd_rn(bmin[a], bmax[a]));
-                        const float r = rintf(__fmul_rn(__fsub_rn(cn, gc[a]), inv_box));
-                        sh[a] = __fmul_rn(p.box, r);
-                        code |= (static_cast<int>(r) + 1) << (2 * a);
-                    }
-                    if (amb)
-                        code = kPerPairImage;
-                }
-                bool pruned = false;
-                if (PERIODIC && amb) {
-                    if (info < 0)
-                        leaf = true;
-                    else
-                        nch = info;
-                } else if (cut) {
-                    float d2 = 0.0f;
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const float lo = __fsub_rn(bmin[a], sh[a]), hi = __fsub_rn(bmax[a], sh[a]);
-                        const float d = fmaxf(fmaxf(__fsub_rn(lo, gmax[a]), __fsub_rn(gmin[a], hi)), 0.0f);
-                        d2 = __fadd_rn(d2, __fmul_rn(d, d));
-                    }
-                    pruned = d2 > p.rcut2;
-                }
-                if (!pruned && !(PERIODIC && amb)) {
-                    float l = 0.0f;
-#pragma unroll
-                    for (int a = 0; a < 3; ++a)
-                        l = fmaxf(l, __fsub_rn(bmax[a], bmin[a]));
-                    // The split kernel varies on the scale r_s, so its expansion error depends on
-                    // the node size itself, not only on l/d: nodes at least max_node_size large
-                    // are never accepted.
-                    const bool small = !capped || l < p.max_node_size;
-                    if (small) {
-                        if (capped)
-                            mo = t.mono[k];
-                        const float com[3] = {mo.x, mo.y, mo.z};
-                        float e2 = 0.0f;
+                bool accept = false, leaf = false, sure = false;
+                int nch = 0, link = 0, info = 0, code = 0;
+                if (k >= 0) {
+                    const float4 b0 = t.box0[k];
+                    const float4 b1 = t.box1[k];
+                    // the centre of mass matters only to a node that may be accepted; with a node
+                    // size cap (TreePM) most nodes are too large, and skip the load
+                    const bool capped = SPLIT && p.max_node_size > 0.0f;  // the cap is a TreePM setting
+                    float4 mo = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (!capped)
+                        mo = t.mono[k];
+                    link = __float_as_int(b0.w);
+                    info = __float_as_int(b1.w);
+                    const float bmin[3] = {b0.x, b0.y, b0.z}, bmax[3] = {b1.x, b1.y, b1.z};
+                    float sh[3] = {0.0f, 0.0f, 0.0f};
+                    bool amb = false;
+                    if (PERIODIC) {
+                        // Image-ambiguous node (its extent + the group's + the cutoff reaches half
+                        // the box): always opened; a leaf is summed with per-pair minimum images.
 #pragma unroll
                         for (int a = 0; a < 3; ++a) {
-                            const float c = __fsub_rn(com[a], sh[a]);
-                            const float e = fmaxf(fmaxf(__fsub_rn(gmin[a], c), __fsub_rn(c, gmax[a])), 0.0f);
-                            e2 = __fadd_rn(e2, __fmul_rn(e, e));
+                            const float nh = __fmul_rn(0.5f, __fsub_rn(bmax[a], bmin[a]));
+                            if (__fadd_rn(__fadd_rn(ghalf[a], nh), rcut) > half_box)
+                                amb = true;
                         }
-                        accept = __fmul_rn(l, l) < __fmul_rn(p.theta2, e2);
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) {
+                            const float cn = __fmul_rn(0.5f, __fadd_rn(bmin[a], bmax[a]));
+                            const float r = rintf(__fmul_rn(__fsub_rn(cn, gc[a]), inv_box));
+                            sh[a] = __fmul_rn(p.box, r);
+                            code |= (static_cast<int>(r) + 1) << (2 * a);
+                        }
+                        if (amb)
+                            code = kPerPairImage;
                     }
-                    if (!accept) {
+                    bool pruned = false;
+                    if (PERIODIC && amb) {
                         if (info < 0)
                             leaf = true;
                         else
                             nch = info;
+                    } else if (cut) {
+                        float d2 = 0.0f;
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) {
+                            const float lo = __fsub_rn(bmin[a], sh[a]), hi = __fsub_rn(bmax[a], sh[a]);
+                            const float d = fmaxf(fmaxf(__fsub_rn(lo, gmax[a]), __fsub_rn(gmin[a], hi)), 0.0f);
+                            d2 = __fadd_rn(d2, __fmul_rn(d, d));
+                        }
+                        pruned = d2 > p.rcut2;
+                    }
+                    if (!pruned && !(PERIODIC && amb)) {
+                        float l = 0.0f;
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+                            l = fmaxf(l, __fsub_rn(bmax[a], bmin[a]));
+                        // The split kernel varies on the scale r_s, so its expansion error depends on
+                        // the node size itself, not only on l/d: nodes at least max_node_size large
+                        // are never accepted.
+                        const bool small = !capped || l < p.max_node_size;
+                        if (small) {
+                            if (capped)
+                                mo = t.mono[k];
+                            const float com[3] = {mo.x, mo.y, mo.z};
+                            float e2 = 0.0f;
+#pragma unroll
+                            for (int a = 0; a < 3; ++a) {
+                                const float c = __fsub_rn(com[a], sh[a]);
+                                const float e = fmaxf(fmaxf(__fsub_rn(gmin[a], c), __fsub_rn(c, gmax[a])), 0.0f);
+                                e2 = __fadd_rn(e2, __fmul_rn(e, e));
+                            }
+                            accept = __fmul_rn(l, l) < __fmul_rn(p.theta2, e2);
+                        }
+                        if (!accept) {
+                            if (info < 0) {
+                                leaf = true;
+                                if (SLICED && sort_leaves) {
+                                    float m2 = 0.0f;
+#pragma unroll
+                                    for (int a = 0; a < 3; ++a) {
+                                        const float lo = bmin[a] - sh[a], hi = bmax[a] - sh[a];
+                                        const float m = fmaxf(hi - gmin[a], gmax[a] - lo);
+                                        m2 = fmaf(m, m, m2);
+                                    }
+                                    sure = m2 <= sure2;
+                                }
+                            } else {
+                                nch = info;
+                            }
+                        }
                     }
                 }
-            }
-            const unsigned am = __ballot_sync(kFullMask, accept);
-            const unsigned lm = __ballot_sync(kFullMask, leaf);
-            if (accept)
-                w.nlist[nn + __popc(am & lt)] = k | (code << kIndexBits);
-            if (leaf) {
-                const int pos = nl + __popc(lm & lt);
-                w.lstart[pos] = link;
-                w.lnode[pos] = k;
-                w.lcount[pos] = -info;
-                w.lcode[pos] = code;
-            }
-            nn += __popc(am);
-            nl += __popc(lm);
-            int lsum = leaf ? -info : 0;
-            for (int off = 16; off > 0; off >>= 1)
-                lsum += __shfl_xor_sync(kFullMask, lsum, off);
-            lp += lsum;
-            cnt_pp += static_cast<unsigned long long>(lsum);
-            cnt_pn += static_cast<unsigned long long>(__popc(am));
-            const int incl = warp_incl_scan(nch);
-            const int tot = __shfl_sync(kFullMask, incl, 31);
-            if (top + tot > kStack) {  // spill the oldest half (uniform branch)
-                const int half = kStack / 2;
-                if (gtop + half > kSpill) {
-                    if (lane == 0)
-                        raise_error(err, kErrWalkStack);
-                    bail = true;
-                    break;
+                const unsigned am = __ballot_sync(kFullMask, accept);
+                const unsigned lm = __ballot_sync(kFullMask, leaf);
+                if (accept)
+                    w.nlist[nn + __popc(am & lt)] = k | (code << kIndexBits);
+                unsigned lmf = lm;
+                if (SLICED && sort_leaves)
+                    lmf = lm & ~__ballot_sync(kFullMask, sure);
+                if (leaf) {
+                    const unsigned mine = sure ? lm & ~lmf : lmf;
+                    const int at = __popc(mine & lt);
+                    const int pos = sure ? kList - 1 - ns - at : nl + at;
+                    w.lstart[pos] = link;
+                    w.lnode[pos] = k;
+                    w.lcount[pos] = -info;
+                    w.lcode[pos] = code;
                 }
-                for (int i = lane; i < half; i += 32)
-                    spill[gtop + i] = w.stack[i];
+                nn += __popc(am);
+                cnt_pn += __popc(am);
+                if (lm != 0u) {
+                    const unsigned lsum = __reduce_add_sync(kFullMask, leaf ? static_cast<unsigned>(-info) : 0u);
+                    nl += __popc(lmf);
+                    ns += __popc(lm & ~lmf);
+                    lp += static_cast<int>(lsum);
+                    cnt_pp += lsum;
+                }
+                const unsigned om = __ballot_sync(kFullMask, nch > 0);
+                const int opened = __popc(om);
+                if (top + opened > kStack) {  // spill the oldest half (uniform branch)
+                    const int half = kStack / 2;
+                    if (gtop + half > kSpill) {
+                        if (lane == 0)
+                            raise_error(err, kErrWalkStack);
+                        break;
+                    }
+                    for (int i = lane; i < half; i += 32)
+                        spill[gtop + i] = static_cast<int>(w.stack[i]);
+                    __syncwarp();
+                    for (int i = lane; i < top - half; i += 32)
+                        w.stack[i] = w.stack[i + half];
+                    __syncwarp();
+                    gtop += half;
+                    top -= half;
+                }
+                if (nch > 0)
+                    w.stack[top + __popc(om & lt)] =
+                        static_cast<unsigned>(link) | static_cast<unsigned>(nch - 1) << kIndexBits;
+                top += opened;
                 __syncwarp();
-                for (int i = lane; i < top - half; i += 32)
-                    w.stack[i] = w.stack[i + half];
+            }
+            if (nn >= (done ? 1 : kNodes)) {
+                const int m = min(nn, kNodes);
+                flush_nodes<PERIODIC, SPLIT, QUAD, POT>(w, m, t, p, inv2rs, lanes, acc);
+                nn -= m;  // the entries past a whole batch (fewer than 32) stay listed
+                const int e = w.nlist[kNodes + lane];
                 __syncwarp();
-                gtop += half;
-                top -= half;
+                if (lane < nn)
+                    w.nlist[lane] = e;
+                __syncwarp();
             }
-            for (int c = 0; c < nch; ++c)
-                w.stack[top + incl - nch + c] = link + c;
-            top += tot;
-            __syncwarp();
-            if (nn >= 32) {
-                flush_nodes<PERIODIC, SPLIT, QUAD, POT>(w, nn, t, p, inv2rs, me.x, me.y, me.z, acc);
-                nn = 0;
+            if (nl + ns >= (done ? 1 : 32) || lp >= kFlushParticles) {
+#pragma unroll 1
+                for (int part = 0; part < (SLICED ? 2 : 1); ++part) {
+                    const int cnt = part ? ns : nl;
+                    if (cnt > 0)
+                        flush_leaves<PERIODIC, SPLIT, POT, SLICED>(
+                            w, part ? kList - ns : 0, cnt, part != 0, pos4, t, p, inv2rs, cut, me.x, me.y,
+                            me.z, ti, acc, phase, err, o, valid ? ti : -1, npair, evald, lanes);
+                }
+                nl = ns = lp = 0;
             }
-            if (nl >= 32 || lp >= kFlushParticles) {
-                flush_leaves<PERIODIC, SPLIT, POT>(w, nl, pos4, t, p, inv2rs, cut, me.x, me.y, me.z,
-                                                   ti, acc, phase, err, o, valid ? ti : -1, npair,
-                                                   evald);
-                nl = 0;
-                lp = 0;
-            }
-        }
-        if (!bail) {
-            if (nn > 0)
-                flush_nodes<PERIODIC, SPLIT, QUAD, POT>(w, nn, t, p, inv2rs, me.x, me.y, me.z, acc);
-            if (nl > 0)
-                flush_leaves<PERIODIC, SPLIT, POT>(w, nl, pos4, t, p, inv2rs, cut, me.x, me.y, me.z,
-                                                   ti, acc, phase, err, o, valid ? ti : -1, npair,
-                                                   evald);
+            if (done && nn == 0)
+                break;
         }
         if (valid) {
             // the walk's sum is clamped, and so is its sum with a mesh force already in the
@@ -872,8 +1245,8 @@ __global__ void __launch_bounds__(kWarps * 32) k_walk(const float4* __restrict__
                 o.n_pn[g] = cnt_pn;
             if (o.totals) {
                 const unsigned long long ng = static_cast<unsigned long long>(gn);
-                atomicAdd(&o.totals[0], cnt_pp * ng);
-                atomicAdd(&o.totals[1], cnt_pn * ng);
+                atomicAdd(&o.totals[0], ng * cnt_pp);
+                atomicAdd(&o.totals[1], ng * cnt_pn);
                 atomicAdd(&o.totals[2], ev);
             }
         }
@@ -899,7 +1272,7 @@ WalkLaunch walk_shape(int n, int blocks_per_sm)
     WalkLaunch local;
     WalkLaunch& c = (dev >= 0 && dev < kMaxDevices) ? cached[dev] : local;
     if (c.blocks == 0) {
-        const size_t smem = sizeof(WarpSmem) * kWarps;
+        const size_t smem = sizeof(WarpSmem<QUAD>) * kWarps;
         cudaFuncSetAttribute(k_walk<PERIODIC, SPLIT, QUAD, POT>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         int sms = 148, per_sm = 1;
