@@ -280,7 +280,7 @@ void enqueue_forces(bz_handle* h, bool kick, bool want_pot, bool mesh_forked = f
     }
     record(h, kPhTree);
     const int root_level = h->systems > 0 ? kSystemLevels : 0;
-    launch_tree_build(d.keys, d.pos4, n, h->cfg.leaf_capacity, kMaxLevels, h->tree, d.err,
+    launch_tree_build(d.keys, d.pos4, n, h->cfg.leaf_capacity, h->tree, d.err,
                       h->stream, root_level, h->cfg.multipole_order >= 2);
     launch_groups(h->tree, n, h->cfg.walk_group_size, root_level, d.keys, h->groups, h->stream);
     record(h, kPhMesh);
@@ -390,8 +390,6 @@ bz_status check_device(bz_handle* h, const char* what)
             m += " radix-sort look-back wait limit reached;";
         if (err & kErrTreeCapacity)
             m += " octree node capacity exceeded;";
-        if (err & kErrTreeSpin)
-            m += " octree look-back wait limit reached;";
         if (err & kErrBulkWait)
             m += " bulk-copy wait limit reached;";
         if (err & kErrListCapacity)
@@ -709,10 +707,9 @@ bz_status bz_create(const bz_config* cfg, size_t capacity, bz_handle** out)
     const size_t cap = static_cast<size_t>(t.cap);
     ok = ok && dalloc(h, &t.start, cap) && dalloc(h, &t.count, cap) && dalloc(h, &t.child, cap) &&
          dalloc(h, &t.nchild, cap) && dalloc(h, &t.parent, cap) && dalloc(h, &t.level, cap) &&
-         dalloc(h, &t.lvl_first, kMaxLevels + 2) && dalloc(h, &t.lvl_count, kMaxLevels + 2) &&
-         dalloc(h, &t.lvl_split, kMaxLevels + 2) &&
-         dalloc(h, &t.n_nodes, 1) && dalloc(h, &t.ticket, kMaxLevels + 2) &&
-         dalloc(h, &t.lookback, tree_lookback_words(t.cap)) && dalloc(h, &t.arrive, cap) &&
+         dalloc(h, &t.lvl_count, kMaxLevels + 1) && dalloc(h, &t.n_nodes, 1) &&
+         dalloc(h, &t.chain, n) && dalloc(h, &t.counts, tree_count_words(static_cast<int>(n))) &&
+         dalloc(h, &t.arrive, cap) &&
          dalloc(h, &t.m64, cap) && dalloc(h, &t.s64, 3 * cap) && dalloc(h, &t.c64, 3 * cap) &&
          dalloc(h, &t.q64, 6 * cap) && dalloc(h, &t.box0, cap) && dalloc(h, &t.box1, cap) &&
          dalloc(h, &t.mono, cap) && dalloc(h, &t.quadA, cap) && dalloc(h, &t.quadB, cap);
@@ -1526,7 +1523,7 @@ bz_status adaptive_steps(bz_handle* h, double dt, uint32_t nsteps)
             if (sub == 0) {
                 enqueue_order(h);
                 record(h, kPhTree);
-                launch_tree_build(d.keys, d.pos4, n, h->cfg.leaf_capacity, kMaxLevels, h->tree, d.err,
+                launch_tree_build(d.keys, d.pos4, n, h->cfg.leaf_capacity, h->tree, d.err,
                                   h->stream, root_level, h->cfg.multipole_order >= 2);
                 launch_groups(h->tree, n, h->cfg.walk_group_size, root_level, d.keys, h->groups,
                               h->stream);

@@ -11,7 +11,6 @@ enum DeviceError : int {
     kErrWalkStack = 1,      // group walk traversal stack would overflow
     kErrSortSpin = 2,       // radix-sort look-back gave up waiting for a predecessor tile
     kErrTreeCapacity = 4,   // more octree nodes than the preallocated capacity
-    kErrTreeSpin = 8,       // octree level look-back gave up waiting
     kErrBulkWait = 16,      // a bulk-copy or MMA mbarrier wait ran out of time
     kErrListCapacity = 32,  // an interaction list exceeded its shared-memory capacity
 };

@@ -97,13 +97,11 @@ struct TreeArrays {
     int* nchild;
     int* parent;
     int* level;
-    int* lvl_first;    // [kMaxLevels+2]
-    int* lvl_count;    // [kMaxLevels+2]
-    int* lvl_split;    // [kMaxLevels+2] 1 when some node of the level holds more than a leaf
+    int* lvl_count;    // [kMaxLevels+1] nodes of each level
     int* n_nodes;      // [1]
-    uint32_t* ticket;  // [kMaxLevels+2]
+    unsigned short* chain;  // [n] levels of the nodes that start at each particle
+    int* counts;       // [tree_count_words(n)] nodes per level and block
     int* arrive;       // [cap] bottom-up arrival counters of the moments climb
-    unsigned long long* lookback;  // [tree_lookback_words(cap)]
     double* m64;       // [cap] FP64 mass
     double* s64;       // [3*cap] FP64 first moments
     double* c64;       // [3*cap] FP64 centre of mass
@@ -117,11 +115,11 @@ struct TreeArrays {
 constexpr int kMaxLevels = 21;
 // Upper bound on device ordinals for per-device caches (function attributes, launch shapes).
 constexpr int kMaxDevices = 64;
-size_t tree_lookback_words(int cap);
+size_t tree_count_words(int n);
 // min_split: nodes above this level split even when small (ensembles use kSystemLevels)
 // quad = false: second moments left zero (walks without quadrupoles)
 void launch_tree_build(const unsigned long long* sorted_keys, const float4* pos4, int n,
-                       int leaf_cap, int max_level, TreeArrays& t, int* err, cudaStream_t s,
+                       int leaf_cap, TreeArrays& t, int* err, cudaStream_t s,
                        int min_split = 0, bool quad = true);
 
 // Keep the topology, recompute every node's tight box and moments from the current pos4

@@ -1,6 +1,6 @@
-// Adaptive linear octree over Morton-sorted particles: top-down topology (one kernel per
-// level, decoupled look-back over the level's child counts, no host round trip) and a single
-// bottom-up moments kernel (last-arriving child computes its parent).
+// Adaptive linear octree over Morton-sorted particles: the topology of all levels at once (each
+// particle decides from its neighbours' keys which nodes start at it) and a single bottom-up
+// moments kernel (last-arriving child computes its parent).
 //
 // This file is compiled with --fmad=false: the FP64 moment sums must round exactly as written
 // (fixed order, no contraction) so that node moments are bit-identical to the oracle's.
@@ -14,44 +14,160 @@
 #include "bz_common.cuh"
 #include "bz_kernels.h"
 
+#include <algorithm>
+
 namespace bz {
 
 namespace {
 
 constexpr int kThreads = 256;
-constexpr unsigned long long kAgg = 1ull << 30;
-constexpr unsigned long long kPrefix = 2ull << 30;
-constexpr unsigned long long kMask = (1ull << 30) - 1;
+constexpr int kLevels = kMaxLevels + 1;  // levels 0 .. kMaxLevels
 
-__global__ void k_tree_init(TreeArrays t, int n)
+// ---- topology ---------------------------------------------------------------------------
+// A cell of level L is the run of particles whose keys share L octant digits.  It is a node of
+// the tree when its parent cell holds more than a leaf (or lies above min_split).  The nodes that
+// start at particle i therefore form one chain of levels [b, e]:
+//   b = the first level whose cell boundary falls between i - 1 and i;
+//   the node (i, b) exists when the cell of level b - 1 around i holds more than leaf_cap
+//   particles (a backward search of at most leaf_cap keys finds that cell's start, unless the
+//   particle leaf_cap before i still belongs to it);
+//   the chain goes on while the cell itself holds more than a leaf: e - 1 = the digits that
+//   particle i shares with particle i + leaf_cap.
+// So every particle decides alone, and the breadth-first index of a node is its level's offset
+// plus the number of that level's starts before i: a count per level and block, one scan of
+// each level, and an emission.  A kernel a level (binary searches for the octant boundaries of
+// every node, a look-back scan) chained 21 launches of 1 to 38 us.  Topology time, level chain ->
+// this: Plummer 65k 163 -> 22 us, isolated TreePM 1M 390 -> 83 us, Hernquist 4M 680 -> 135 us,
+// the 256^3 lattice 298 -> 314 us (the tree phase with it 0.73 -> 0.67 ms).  Bound by latency below a
+// million particles (four launches), by the issue of the key comparisons above.
+
+// Octant digits two keys share (0 .. kMaxLevels).
+__device__ __forceinline__ int common_levels(unsigned long long x, unsigned long long y)
 {
-    const int i = threadIdx.x;
-    if (i < kMaxLevels + 2) {
-        t.lvl_first[i] = 0;
-        t.lvl_count[i] = 0;
-        t.lvl_split[i] = 0;
-        t.ticket[i] = 0;
-    }
-    if (i == 0) {
-        t.lvl_count[0] = 1;
-        t.lvl_split[0] = 1;  // the root level goes the general way
-        t.n_nodes[0] = 1;
-        t.start[0] = 0;
-        t.count[0] = n;
-        t.parent[0] = -1;
-        t.level[0] = 0;
-        t.arrive[0] = 0;
-    }
+    return x == y ? kMaxLevels : (__clzll(static_cast<long long>(x ^ y)) - 1) / 3;
 }
 
-__device__ __forceinline__ int lower_bound_digit(const unsigned long long* __restrict__ keys,
-                                                 int lo, int hi, int shift, unsigned d)
+// Whether two keys share l octant digits.
+__device__ __forceinline__ bool shares(unsigned long long x, unsigned long long y, int l)
 {
-    // first i in [lo, hi) with digit(i) >= d (digits are non-decreasing inside a cell)
+    return ((x ^ y) >> (3 * (kMaxLevels - l))) == 0ull;
+}
+
+// Particles a thread takes, by the system's size: short runs fill the SMs with the smaller
+// systems, long ones keep the scan of the block counts short.
+constexpr int kTreeSmall = 1 << 20, kTreeMiddle = 1 << 23;
+int tree_items(int n) { return n < kTreeSmall ? 2 : (n < kTreeMiddle ? 4 : 16); }
+int tree_blocks(int n) { return (n + kThreads * tree_items(n) - 1) / (kThreads * tree_items(n)); }
+
+// The boundary level b and the chain [b, e] of every particle (packed b | e << 8; e < b where no
+// node starts) and, per level and block, the nodes.
+__global__ void __launch_bounds__(kThreads) k_tree_chains(const unsigned long long* __restrict__ keys, int n,
+                                                           int items, int leaf_cap, int min_split,
+                                                           unsigned short* __restrict__ chain,
+                                                           int* __restrict__ counts)
+{
+    __shared__ int cnt[kLevels];
+    if (threadIdx.x < kLevels)
+        cnt[threadIdx.x] = 0;
+    __syncthreads();
+    const int base = blockIdx.x * kThreads * items;
+    const int back = (leaf_cap + 1) / 2, ahead = leaf_cap / 2;
+#pragma unroll 4
+    for (int it = 0; it < items; ++it) {
+        const int i = base + it * kThreads + threadIdx.x;
+        if (i >= n)
+            break;
+        // all the keys that most particles need, loaded side by side
+        const unsigned long long key = keys[i], prev = keys[max(i - 1, 0)];
+        const unsigned long long kb = keys[max(i - back, 0)], ka = keys[ahead < n - i ? i + ahead : i];
+        const unsigned long long kl = keys[max(i - leaf_cap, 0)], kr = keys[leaf_cap < n - i ? i + leaf_cap : i];
+        const int b = i > 0 ? common_levels(prev, key) + 1 : 0;
+        bool exists = b <= min_split;
+        if (!exists && b <= kMaxLevels) {
+            // More than leaf_cap particles around i in one cell reach half a leaf to one side of
+            // it at least (most particles, inside a leaf, stop here).
+            const int l = b - 1;
+            if ((i >= back && shares(kb, key, l)) || (ahead < n - i && shares(ka, key, l))) {
+                if (i >= leaf_cap && shares(kl, key, l)) {
+                    exists = true;
+                } else {
+                    // the start of the cell of level l around i, less than leaf_cap before it
+                    int lo = max(i - leaf_cap + 1, 0), hi = i;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (shares(keys[mid], key, l))
+                            hi = mid;
+                        else
+                            lo = mid + 1;
+                    }
+                    // (leaf_cap may exceed n: no sum before the comparison)
+                    exists = leaf_cap < n - lo && shares(keys[lo + leaf_cap], key, l);
+                }
+            }
+        }
+        int packed = b;  // e = 0 < b: no node starts here
+        if (exists) {
+            int e = max(b, min_split);
+            if (leaf_cap < n - i)
+                e = max(e, min(common_levels(kr, key) + 1, kMaxLevels));
+            packed = b | e << 8;
+            for (int l = b; l <= e; ++l)
+                atomicAdd(&cnt[l], 1);
+        }
+        chain[i] = static_cast<unsigned short>(packed);
+    }
+    __syncthreads();
+    if (threadIdx.x < kLevels)
+        counts[threadIdx.x * gridDim.x + blockIdx.x] = cnt[threadIdx.x];
+}
+
+// Block l: exclusive scan of level l's block counts, its total to lvl_count[l].
+__global__ void __launch_bounds__(1024) k_tree_scan(int* __restrict__ counts, int blocks, TreeArrays t)
+{
+    __shared__ int carry;
+    __shared__ int ws[32];
+    int* c = counts + static_cast<size_t>(blockIdx.x) * blocks;
+    if (threadIdx.x == 0)
+        carry = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int base = 0; base < blocks; base += 1024) {
+        const int i = base + threadIdx.x;
+        const int v = i < blocks ? c[i] : 0;
+        const int x = warp_incl_scan(v);
+        if (lane == 31)
+            ws[warp] = x;
+        __syncthreads();
+        if (warp == 0)
+            ws[lane] = warp_incl_scan(ws[lane]);
+        __syncthreads();
+        const int before = (warp > 0 ? ws[warp - 1] : 0) + carry;
+        if (i < blocks)
+            c[i] = before + x - v;
+        __syncthreads();
+        if (threadIdx.x == 1023)
+            carry = before + x;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0)
+        t.lvl_count[blockIdx.x] = carry;
+}
+
+// First particle after `from` (which shares l digits with key), at most `limit`, that does not.
+__device__ __forceinline__ int cell_end(const unsigned long long* __restrict__ keys, unsigned long long key,
+                                        int from, int l, int limit)
+{
+    int lo = from;
+    int step = 32;
+    while (step < limit - lo && shares(keys[lo + step], key, l)) {
+        lo += step;
+        step <<= 1;
+    }
+    int hi = step < limit - lo ? lo + step : limit;
+    ++lo;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        const unsigned dm = static_cast<unsigned>((keys[mid] >> shift) & 7u);
-        if (dm < d)
+        if (shares(keys[mid], key, l))
             lo = mid + 1;
         else
             hi = mid;
@@ -59,211 +175,114 @@ __device__ __forceinline__ int lower_bound_digit(const unsigned long long* __res
     return lo;
 }
 
-__device__ __forceinline__ unsigned long long vload(const unsigned long long* p)
+// Writes the nodes.  Each warp takes 32 x items consecutive particles, lists those at which nodes
+// start, and works on 32 of these at a time (an eighth of a lattice's particles start a node; with
+// a lane a particle the kernel took 292 us at 16.7M, 98 so).  Lane l of a warp carries
+// the index of level l's next node.  A node ends where the next start with b <= its level lies:
+// every cell boundary that ends a node starts another one, a child of their common ancestor.
+__global__ void __launch_bounds__(kThreads) k_tree_emit(const unsigned long long* __restrict__ keys, int n, int items,
+                                                         const unsigned short* __restrict__ chain,
+                                                         const int* __restrict__ counts, TreeArrays t, int* err)
 {
-    return *reinterpret_cast<const volatile unsigned long long*>(p);
-}
-__device__ __forceinline__ void vstore(unsigned long long* p, unsigned long long v)
-{
-    *reinterpret_cast<volatile unsigned long long*>(p) = v;
-}
-
-// Split every node of level `l` with more than leaf_cap particles into its non-empty octant
-// cells.  Children of the level are appended in (parent, octant) order.  On the top levels
-// (few, very large nodes) TPN = 8 threads serve one node: thread d (1..7) finds the first
-// particle whose digit is >= d, so the seven binary searches run side by side; deeper levels
-// use one thread per node.  Look-back tiles are indexed in units of kLookbackNodes nodes.
-constexpr int kLookbackNodes = kThreads / 8;
-
-template <int TPN>
-__global__ void __launch_bounds__(kThreads) k_tree_level(const unsigned long long* __restrict__ keys,
-                                                          int l, int leaf_cap, int max_level,
-                                                          int min_split, TreeArrays t, int* err)
-{
-    constexpr int kNodesPerTile = kThreads / TPN;
-    __shared__ int s_tile;
-    __shared__ int s_scan[kThreads / 32];
-    __shared__ int s_prefix;
-    const int first = t.lvl_first[l];
-    const int level_splits = t.lvl_split[l];  // loaded with the level's range, one round trip
-    // after a capacity overflow the recorded count can exceed the arrays: clamp
-    const int cnt = min(t.lvl_count[l], t.cap - first);
-    if (cnt <= 0)
-        return;
-    const int next_first = first + cnt;
-    if (level_splits == 0 && l >= min_split) {
-        // no node of this level holds more than a leaf: all are leaves, no children, no scan
-        for (int i = blockIdx.x * kThreads + threadIdx.x; i < cnt; i += gridDim.x * kThreads) {
-            t.child[first + i] = -1;
-            t.nchild[first + i] = 0;
+    extern __shared__ int s_list[];  // [kThreads * items]: offset | b << 16 | e << 24
+    __shared__ int ws[kThreads / 32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lt = lanemask_lt();
+    // level offsets; levels that would pass the node capacity are cut off: the nodes of the last
+    // level kept stay leaves, and the overflow is reported
+    const int total = lane < kLevels ? t.lvl_count[lane] : 0;
+    const long long incl = [&] {
+        long long x = total;
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(kFullMask, x, o);
+            if (lane >= o)
+                x += y;
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            t.lvl_first[l + 1] = next_first;
-            t.lvl_count[l + 1] = 0;
-            t.n_nodes[0] = min(next_first, t.cap);
-        }
-        return;
+        return x;
+    }();
+    const unsigned fits = __ballot_sync(kFullMask, lane < kLevels && incl <= t.cap);
+    const int last = 31 - __clz(fits);  // (level 0 holds one node: it always fits)
+    const int nodes = static_cast<int>(__shfl_sync(kFullMask, incl, last));
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        t.n_nodes[0] = nodes;
+        t.parent[0] = -1;
+        if (last < kMaxLevels)
+            raise_error(err, kErrTreeCapacity);
     }
-    const int ntiles = (cnt + kNodesPerTile - 1) / kNodesPerTile;
-    unsigned long long* lb = t.lookback + (first / kLookbackNodes + 2 * l);
-    const int shift = 3 * (max_level - l - 1);
-    const int slot = threadIdx.x / TPN, sub = threadIdx.x % TPN, lane = threadIdx.x & 31;
-    for (;;) {
-        if (threadIdx.x == 0)
-            s_tile = static_cast<int>(atomicAdd(&t.ticket[l], 1u));
-        __syncthreads();
-        const int tile = s_tile;
-        __syncthreads();
-        if (tile >= ntiles)
-            break;
-        const int k = first + tile * kNodesPerTile + slot;
-        int s0 = 0, c0 = 0;
-        bool split = false;
-        int bsub = 0;
-        int b[9];
-        if (k < next_first) {
-            s0 = t.start[k];
-            c0 = t.count[k];
-            // levels above min_split always split (ensembles: they separate the systems)
-            split = (c0 > leaf_cap || l < min_split) && l < max_level;
-            if (TPN == 8) {
-                if (split && sub > 0)
-                    bsub = lower_bound_digit(keys, s0, s0 + c0, shift, static_cast<unsigned>(sub));
-            } else if (split) {
-                // the seven searches advance in lockstep, so each step's seven loads are in
-                // flight together (one memory round trip per step, not one per search step)
-                int lo[8], hi[8];
-#pragma unroll
-                for (int d = 1; d < 8; ++d) {
-                    lo[d] = s0;
-                    hi[d] = s0 + c0;
-                }
-                for (int step = 0; step < 32; ++step) {
-                    bool open = false;
-#pragma unroll
-                    for (int d = 1; d < 8; ++d) {
-                        if (lo[d] < hi[d]) {
-                            const int mid = (lo[d] + hi[d]) >> 1;
-                            const unsigned dm = static_cast<unsigned>((keys[mid] >> shift) & 7u);
-                            if (dm < static_cast<unsigned>(d))
-                                lo[d] = mid + 1;
-                            else
-                                hi[d] = mid;
-                            open = true;
-                        }
-                    }
-                    if (!open)
-                        break;
-                }
-#pragma unroll
-                for (int d = 1; d < 8; ++d)
-                    b[d] = lo[d];
-            }
+    const int base = (blockIdx.x * (kThreads / 32) + warp) * 32 * items;
+    int* list = s_list + warp * 32 * items;
+    int starts = 0;
+    for (int r = 0; r < items; ++r) {
+        const int i = base + r * 32 + lane;
+        const int c = i < n ? chain[i] : 1;
+        const int b = c & 0xff, e = min(c >> 8, last);
+        const unsigned m = __ballot_sync(kFullMask, b <= e);
+        if (b <= e)
+            list[starts + __popc(m & lt)] = (r * 32 + lane) | b << 16 | e << 24;
+        starts += __popc(m);
+    }
+    __syncwarp();
+    int mine = 0;
+    for (int g = 0; g < starts; g += 32) {
+        const int c = g + lane < starts ? list[g + lane] : 1 << 16;
+        const int b = c >> 16 & 0xff, e = c >> 24;
+        const int lo = __reduce_min_sync(kFullMask, b <= e ? b : kLevels), hi = __reduce_max_sync(kFullMask, b <= e ? e : -1);
+        for (int l = lo; l <= hi; ++l) {
+            const int k = __popc(__ballot_sync(kFullMask, b <= l && l <= e));
+            mine += lane == l ? k : 0;
         }
-        if (TPN == 8) {
-#pragma unroll
-            for (int d = 1; d < 8; ++d)
-                b[d] = __shfl_sync(kFullMask, bsub, (lane & ~7) + d);
-        }
-        b[0] = s0;
-        b[8] = s0 + c0;
-        int nch = 0;
-        if (split && sub == 0) {
-#pragma unroll
-            for (int d = 0; d < 8; ++d)
-                nch += b[d + 1] > b[d] ? 1 : 0;
-        }
-        // block scan of child counts (only the leader of each node contributes): warp scans,
-        // then one warp scans the warp totals
-        const int wincl = warp_incl_scan(nch);
-        const int warp = threadIdx.x >> 5;
-        if (lane == 31)
-            s_scan[warp] = wincl;
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            int v = threadIdx.x < kThreads / 32 ? s_scan[threadIdx.x] : 0;
-            v = warp_incl_scan(v);
-            if (threadIdx.x < kThreads / 32)
-                s_scan[threadIdx.x] = v;
-        }
-        __syncthreads();
-        const int incl = wincl + (warp > 0 ? s_scan[warp - 1] : 0);
-        const int total = s_scan[kThreads / 32 - 1];
-        if (threadIdx.x == 0) {
-            unsigned long long excl = 0;
-            if (tile == 0) {
-                vstore(&lb[0], kPrefix | static_cast<unsigned long long>(total));
-            } else {
-                vstore(&lb[tile], kAgg | static_cast<unsigned long long>(total));
-                int tt = tile - 1, spins = 0;
-                while (tt >= 0) {
-                    const unsigned long long v = vload(&lb[tt]);
-                    if ((v & (3ull << 30)) == 0) {
-                        if (++spins > kSpinLimit) {
-                            raise_error(err, kErrTreeSpin);
-                            break;
-                        }
-                        if (spins > 32)
-                            __nanosleep(32);
-                        continue;
-                    }
-                    excl += v & kMask;
-                    if (v & kPrefix)
-                        break;
-                    --tt;
-                }
-                vstore(&lb[tile], kPrefix | (excl + static_cast<unsigned long long>(total)));
-            }
-            s_prefix = static_cast<int>(excl);
-            if (tile == ntiles - 1) {
-                const int children = static_cast<int>(excl) + total;
-                t.lvl_first[l + 1] = next_first;
-                t.lvl_count[l + 1] = children;
-                t.n_nodes[0] = min(next_first + children, t.cap);
-                if (next_first + children > t.cap)
-                    raise_error(err, kErrTreeCapacity);
-            }
-        }
-        __syncthreads();
-        int cmax = 0;
-        if (k < next_first && sub == 0) {
-            int c = next_first + s_prefix + incl - nch;
-            if (split && c + nch > t.cap)
-                nch = 0;  // capacity exceeded (error raised above): keep the node a leaf
-            t.child[k] = nch > 0 ? c : -1;
-            t.nchild[k] = nch;
-            if (nch > 0) {
-#pragma unroll
-                for (int d = 0; d < 8; ++d) {
-                    if (b[d + 1] > b[d]) {
-                        t.start[c] = b[d];
-                        t.count[c] = b[d + 1] - b[d];
-                        t.parent[c] = k;
-                        t.level[c] = l + 1;
-                        t.arrive[c] = 0;
-                        cmax = max(cmax, b[d + 1] - b[d]);
-                        ++c;
-                    }
+    }
+    ws[warp][lane] = mine;
+    __syncthreads();
+    int next = static_cast<int>(incl) - total;
+    if (lane < kLevels)
+        next += counts[static_cast<size_t>(lane) * gridDim.x + blockIdx.x];
+    for (int w = 0; w < warp; ++w)
+        next += ws[w][lane];
+    for (int g = 0; g < starts; g += 32) {
+        const bool real = g + lane < starts;
+        const int c = real ? list[g + lane] : 1 << 16;
+        const int i = base + (c & 0xffff), b = c >> 16 & 0xff, e = c >> 24;
+        const int lo = __reduce_min_sync(kFullMask, b <= e ? b : kLevels), hi = __reduce_max_sync(kFullMask, b <= e ? e : -1);
+        const int tail = __shfl_sync(kFullMask, i, min(starts - g, 32) - 1);  // the last start here
+        const unsigned long long key = real ? keys[i] : 0ull;
+        // the node of the level above that starts last before this particle
+        int above = lo > 0 ? __shfl_sync(kFullMask, next, lo - 1) - 1 : -1;
+        int end = n;
+        for (int l = lo; l <= hi; ++l) {
+            const bool in = b <= l && l <= e;
+            const unsigned m = __ballot_sync(kFullMask, in);
+            const unsigned edge = __ballot_sync(kFullMask, real && b <= l) & (0xfffffffeu << lane);
+            const int at = __shfl_sync(kFullMask, i, edge != 0u ? __ffs(edge) - 1 : 0);
+            const int k = __shfl_sync(kFullMask, next, l) + __popc(m & lt);
+            if (in) {
+                end = edge != 0u ? at : (l == 0 ? n : cell_end(keys, key, tail, l, end));
+                t.start[k] = i;
+                t.count[k] = end - i;
+                t.parent[k] = above;
+                t.level[k] = l;
+                t.arrive[k] = 0;
+                if (l > b)
+                    t.child[above] = k;  // the chain's node above starts at this particle too
+                if (l == e) {
+                    t.child[k] = -1;
+                    t.nchild[k] = 0;
                 }
             }
+            above = in ? k : k - 1;
+            next += lane == l ? __popc(m) : 0;
         }
-        // a child larger than a leaf lets the next level split: flag it (plain stores of the
-        // same value, which no thread waits for, instead of contended atomics)
-        if (__any_sync(kFullMask, cmax > leaf_cap) && lane == 0)
-            t.lvl_split[l + 1] = 1;
-        __syncthreads();
     }
 }
 
-// Leaves of the deepest level are never visited by k_tree_level (it stops at max_level), so
-// their child fields are written here before the moments pass reads them.
-__global__ void k_tree_finish_last(TreeArrays t, int max_level)
+// The child count of every split node, from the last of its (consecutive) children.
+__global__ void __launch_bounds__(kThreads) k_tree_children(TreeArrays t)
 {
-    const int first = t.lvl_first[max_level];
-    const int cnt = min(t.lvl_count[max_level], t.cap - first);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x) {
-        t.child[first + i] = -1;
-        t.nchild[first + i] = 0;
+    const int nn = t.n_nodes[0];
+    for (int k = blockIdx.x * kThreads + threadIdx.x + 1; k < nn; k += gridDim.x * kThreads) {
+        const int p = t.parent[k];
+        if (k + 1 == nn || t.parent[k + 1] != p)
+            t.nchild[p] = k - t.child[p] + 1;
     }
 }
 
@@ -441,41 +460,26 @@ void launch_tree_refit(const float4* pos4, TreeArrays& t, cudaStream_t s, bool q
     enqueue_moments(pos4, t, sms, s, quad, true);
 }
 
-size_t tree_lookback_words(int cap) { return static_cast<size_t>(cap) / kLookbackNodes + 2 * kMaxLevels + 8; }
+size_t tree_count_words(int n)
+{
+    // the largest of any n' <= n: a workspace serves every smaller system
+    const int a = tree_blocks(std::min(n, kTreeSmall - 1)), b = tree_blocks(std::min(n, kTreeMiddle - 1));
+    return static_cast<size_t>(std::max(tree_blocks(n), std::max(a, b))) * kLevels;
+}
 
-void launch_tree_build(const unsigned long long* sorted_keys, const float4* pos4, int n,
-                       int leaf_cap, int max_level, TreeArrays& t, int* err, cudaStream_t s,
-                       int min_split, bool quad)
+void launch_tree_build(const unsigned long long* sorted_keys, const float4* pos4, int n, int leaf_cap,
+                       TreeArrays& t, int* err, cudaStream_t s, int min_split, bool quad)
 {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaMemsetAsync(t.lookback, 0, tree_lookback_words(t.cap) * sizeof(unsigned long long), s);
-    count_launch();
-    k_tree_init<<<1, 32, 0, s>>>(t, n);
-    // Level l holds at most min(8^l, n) nodes; the persistent grid covers that with tiles.
-    for (int l = 0; l < max_level; ++l) {
-        long long bound = 1;
-        for (int j = 0; j < l && bound < n; ++j)
-            bound *= 8;
-        if (bound > n)
-            bound = n;
-        const bool wide = bound <= 4096;  // top levels: few, large nodes
-        const long long per_tile = wide ? kThreads / 8 : kThreads;
-        long long blocks = (bound + per_tile - 1) / per_tile;
-        // the tiles are latency-bound (loads, scan, look-back): fill the SMs (8 blocks each)
-        if (blocks > 8LL * sms)
-            blocks = 8LL * sms;
-        count_launch();
-        if (wide)
-            k_tree_level<8><<<static_cast<int>(blocks), kThreads, 0, s>>>(sorted_keys, l, leaf_cap,
-                                                                          max_level, min_split, t, err);
-        else
-            k_tree_level<1><<<static_cast<int>(blocks), kThreads, 0, s>>>(sorted_keys, l, leaf_cap,
-                                                                          max_level, min_split, t, err);
-    }
-    count_launch();
-    k_tree_finish_last<<<sms, 256, 0, s>>>(t, max_level);
+    const int items = tree_items(n), blocks = tree_blocks(n);
+    count_launch(4);
+    k_tree_chains<<<blocks, kThreads, 0, s>>>(sorted_keys, n, items, leaf_cap, min_split, t.chain, t.counts);
+    k_tree_scan<<<kLevels, 1024, 0, s>>>(t.counts, blocks, t);
+    k_tree_emit<<<blocks, kThreads, sizeof(int) * kThreads * items, s>>>(sorted_keys, n, items, t.chain, t.counts, t, err);
+    const int cb = (n + kThreads - 1) / kThreads;
+    k_tree_children<<<cb < 8 * sms ? cb : 8 * sms, kThreads, 0, s>>>(t);
     enqueue_moments(pos4, t, sms, s, quad, false);
 }
 
