@@ -27,7 +27,7 @@ constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
 constexpr size_t kMaxKeys = BZ_SORT_NOALLOC_MAX_KEYS;
-constexpr size_t kTileItems = 4096;  // onesweep tile; checked against sort_tile_items()
+constexpr size_t kTileItems = 2048;  // onesweep tile; checked against sort_tile_items()
 constexpr size_t kStateWords = (kMaxKeys + kTileItems - 1) / kTileItems * 256;
 
 constexpr size_t kOffKeys = 0;
@@ -39,7 +39,7 @@ constexpr size_t kOffTicket = align_up(kOffBase + 4 * 8 * 256);
 constexpr size_t kOffEpoch = align_up(kOffTicket + 4 * 8);
 constexpr size_t kOffTrivial = align_up(kOffEpoch + 4);
 constexpr size_t kOffErr = align_up(kOffTrivial + 4 * 8);
-constexpr size_t kScratchBytes = align_up(kOffErr + 4);  // 12.6 MiB for 2^20 keys
+constexpr size_t kScratchBytes = align_up(kOffErr + 4);  // 13.1 MiB for 2^20 keys
 
 // The scratch.  In host code this name is only a host-side stand-in for the symbol: the
 // device address comes from cudaGetSymbolAddress, once per device (scratch_on_device).

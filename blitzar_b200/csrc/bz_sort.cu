@@ -16,8 +16,18 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kIter = 16;                     // keys per lane
-constexpr int kTile = kWarps * 32 * kIter;    // 4096 keys per tile
+// Keys per lane and tile.  Below kShortTileKeys keys the tiles are half as long: a pass is then the
+// time of the one tile an SM takes, not of the memory (whole sorts of 60 thousand pairs 149 ->
+// 130 us, of 300 thousand 170 -> 156 us; of a million no difference); above, long tiles halve the
+// look-back words.
+constexpr int kIterLong = 16, kIterShort = 8;
+constexpr int kShortTileKeys = 1 << 19;
+constexpr int tile_keys(int iter) { return kWarps * 32 * iter; }
+int sort_iter(int n) { return n < kShortTileKeys ? kIterShort : kIterLong; }
+// Predecessors a look-back step reads at once.  The tiles of a pass start together, so late ones
+// look back over many of them; one at a time, that chain of loads was 1.5 of the 22 us of a pass
+// of a million keys.
+constexpr int kLookBatch = 8;
 constexpr unsigned long long kFlagAgg = 1ull << 30;
 constexpr unsigned long long kFlagPrefix = 2ull << 30;
 constexpr unsigned long long kValueMask = (1ull << 30) - 1;
@@ -93,9 +103,9 @@ __device__ __forceinline__ void store_state(unsigned long long* p, unsigned long
     *reinterpret_cast<volatile unsigned long long*>(p) = v;
 }
 
-struct PassSmem {
-    unsigned long long keys[kTile];
-    uint32_t vals[kTile];
+template <int ITER> struct PassSmem {
+    unsigned long long keys[tile_keys(ITER)];
+    uint32_t vals[tile_keys(ITER)];
     uint32_t warp_hist[kWarps][256];
     uint32_t tile_excl[256];
     uint32_t global_off[256];
@@ -103,12 +113,14 @@ struct PassSmem {
     int tile;
 };
 
+template <int ITER>
 __global__ void __launch_bounds__(kThreads) k_onesweep(unsigned long long* keys_a, uint32_t* vals_a,
                                                         unsigned long long* keys_b,
                                                         uint32_t* vals_b, int n, int pass,
                                                         SortWorkspace ws, int* err,
                                                         const SortJob* __restrict__ job)
 {
+    constexpr int kIter = ITER, kTile = tile_keys(ITER);
     if (ws.trivial[pass])
         return;
     if (job) {
@@ -119,7 +131,7 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(unsigned long long* keys_
         n = job->n;
     }
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    PassSmem& sm = *reinterpret_cast<PassSmem*>(smem_raw);
+    PassSmem<ITER>& sm = *reinterpret_cast<PassSmem<ITER>*>(smem_raw);
     int np = 0;
     for (int p = 0; p < pass; ++p)
         np += ws.trivial[p] ? 0 : 1;
@@ -160,7 +172,15 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(unsigned long long* keys_
         const long long idx = base + w * (32 * kIter) + k * 32 + lane;
         const bool valid = idx < n;
         const unsigned d = static_cast<unsigned>((kr[k] >> shift) & 255u);
-        const unsigned peers = __match_any_sync(kFullMask, valid ? d : 256u + lane);
+        // lanes with the same digit, by a vote a bit (a sort of a million pairs takes 209 us so,
+        // 242 us with __match_any_sync)
+        unsigned peers = __ballot_sync(kFullMask, valid);
+#pragma unroll
+        for (int bit = 0; bit < 8; ++bit) {
+            const bool set = (d >> bit) & 1u;
+            const unsigned m = __ballot_sync(kFullMask, set);
+            peers &= set ? m : ~m;
+        }
         if (valid)
             rank[k] = sm.warp_hist[w][d] + __popc(peers & lt);
         __syncwarp();
@@ -188,21 +208,32 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(unsigned long long* keys_
         store_state(&st[static_cast<size_t>(tile) * 256 + d], tag | kFlagAgg | cnt);
         int t = tile - 1;
         int spins = 0;
-        while (t >= 0) {
-            const unsigned long long v = load_state(&st[static_cast<size_t>(t) * 256 + d]);
-            if ((v & 0xffffffff00000000ull) != tag || (v & (3ull << 30)) == 0) {
+        bool found = false;
+        while (t >= 0 && !found) {
+            unsigned long long v[kLookBatch];
+#pragma unroll
+            for (int q = 0; q < kLookBatch; ++q)
+                v[q] = t >= q ? load_state(&st[static_cast<size_t>(t - q) * 256 + d]) : 0ull;
+            bool ready = true;
+            int taken = 0;
+#pragma unroll
+            for (int q = 0; q < kLookBatch; ++q) {
+                ready = ready && !found && (v[q] & 0xffffffff00000000ull) == tag && (v[q] & (3ull << 30)) != 0;
+                if (ready) {
+                    excl += static_cast<uint32_t>(v[q] & kValueMask);
+                    found = (v[q] & kFlagPrefix) != 0;
+                    ++taken;
+                }
+            }
+            t -= taken;
+            if (taken == 0) {
                 if (++spins > kSpinLimit) {
                     raise_error(err, kErrSortSpin);
                     break;
                 }
                 if (spins > 32)
                     __nanosleep(32);
-                continue;
             }
-            excl += static_cast<uint32_t>(v & kValueMask);
-            if (v & kFlagPrefix)
-                break;
-            --t;
         }
         store_state(&st[static_cast<size_t>(tile) * 256 + d], tag | kFlagPrefix | (excl + cnt));
     }
@@ -271,15 +302,49 @@ __global__ void k_fixup(unsigned long long* keys_a, uint32_t* vals_a,
 
 } // namespace
 
-int sort_tile_items() { return kTile; }
+int sort_tile_items() { return tile_keys(kIterShort); }
 
 size_t sort_state_words(int n)
 {
-    const size_t tiles = (static_cast<size_t>(n) + kTile - 1) / kTile;
-    return (tiles < 1 ? 1 : tiles) * 256;
+    // the most tiles of any n' <= n: a workspace serves every smaller sort
+    auto tiles = [](int m) { return (m + tile_keys(sort_iter(m)) - 1) / tile_keys(sort_iter(m)); };
+    const int few = tiles(n), many = tiles(n < kShortTileKeys ? n : kShortTileKeys - 1);
+    const int t = few > many ? few : many;
+    return static_cast<size_t>(t < 1 ? 1 : t) * 256;
 }
 
 namespace {
+
+template <int ITER>
+void enqueue_passes(unsigned long long* keys, uint32_t* vals, int n, int passes, SortWorkspace& ws, int* err,
+                    int dev, int sms, cudaStream_t s, const SortJob* job)
+{
+    const int tiles = (n + tile_keys(ITER) - 1) / tile_keys(ITER);
+    const size_t smem = sizeof(PassSmem<ITER>);
+    // function attributes belong to the device's context: set once per device
+    static std::atomic<bool> attr_set[kMaxDevices];
+    if (dev < 0 || dev >= kMaxDevices || !attr_set[dev].load()) {
+        cudaFuncSetAttribute(k_onesweep<ITER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(smem));
+        if (dev >= 0 && dev < kMaxDevices)
+            attr_set[dev].store(true);
+    }
+    // persistent grid: the resident blocks (at most one per tile)
+    static std::atomic<int> resident[kMaxDevices];
+    int per_sm = dev >= 0 && dev < kMaxDevices ? resident[dev].load() : 0;
+    if (per_sm <= 0) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_onesweep<ITER>, kThreads, smem);
+        per_sm = per_sm > 0 ? per_sm : 1;
+        if (dev >= 0 && dev < kMaxDevices)
+            resident[dev].store(per_sm);
+    }
+    const int grid = tiles < per_sm * sms ? tiles : per_sm * sms;
+    for (int p = 0; p < passes; ++p) {
+        count_launch();
+        k_onesweep<ITER><<<grid, kThreads, smem, s>>>(keys, vals, ws.keys_alt, ws.vals_alt, n, p, ws,
+                                                      err, job);
+    }
+}
 
 // The passes for a grid of capacity n; with `job` the device-held arrays and count decide the
 // work.
@@ -298,31 +363,10 @@ void enqueue_sort(unsigned long long* keys, uint32_t* vals, int n, int bits, Sor
     k_histogram<<<hb, kThreads, 0, s>>>(keys, n, passes, ws, job);
     count_launch();
     k_scan_hist<<<passes, 256, 0, s>>>(n, ws, job);
-    const int tiles = (n + kTile - 1) / kTile;
-    const size_t smem = sizeof(PassSmem);
-    // function attributes belong to the device's context: set once per device
-    static std::atomic<bool> attr_set[kMaxDevices];
-    if (dev < 0 || dev >= kMaxDevices || !attr_set[dev].load()) {
-        cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
-        if (dev >= 0 && dev < kMaxDevices)
-            attr_set[dev].store(true);
-    }
-    // persistent grid: the resident blocks (at most one per tile)
-    static std::atomic<int> resident[kMaxDevices];
-    int per_sm = dev >= 0 && dev < kMaxDevices ? resident[dev].load() : 0;
-    if (per_sm <= 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_onesweep, kThreads, smem);
-        per_sm = per_sm > 0 ? per_sm : 1;
-        if (dev >= 0 && dev < kMaxDevices)
-            resident[dev].store(per_sm);
-    }
-    const int grid = tiles < per_sm * sms ? tiles : per_sm * sms;
-    for (int p = 0; p < passes; ++p) {
-        count_launch();
-        k_onesweep<<<grid, kThreads, smem, s>>>(keys, vals, ws.keys_alt, ws.vals_alt, n, p, ws,
-                                                err, job);
-    }
+    if (sort_iter(n) == kIterShort)
+        enqueue_passes<kIterShort>(keys, vals, n, passes, ws, err, dev, sms, s, job);
+    else
+        enqueue_passes<kIterLong>(keys, vals, n, passes, ws, err, dev, sms, s, job);
     int fb = (n + 255) / 256;
     fb = fb < 4 * sms ? fb : 4 * sms;
     count_launch();
@@ -353,17 +397,24 @@ void launch_radix_sort(unsigned long long* keys, uint32_t* vals, int n, int bits
 // kernels of the path not taken return at once.
 namespace {
 
-constexpr int kInvItems = 16;
-constexpr int kInvChunk = kThreads * kInvItems;  // positions per flag/compaction block
+// Positions per flag/compaction block: kThreads x 16, or x 4 below kInvSmall positions, where
+// long chunks leave most SMs without a block and the chunk's serial loop is the time (65k keys:
+// flags 14.2 -> 4.8 us, split 16.5 -> 5.5 us; at 16.7M the short chunks' scan of 16 thousand block sums
+// would cost more than it saves).
+constexpr int kInvItems = 16, kInvItemsSmall = 4;
+constexpr int kInvSmall = 1 << 20;
+int inv_items(int n) { return n < kInvSmall ? kInvItemsSmall : kInvItems; }
 constexpr int kMergeSeg = 256;                  // in-order positions per merge segment
 constexpr int kWindow = 8;                      // neighbours compared on each side
 
 // Flags the out-of-order positions of a chunk (staged with its halo in shared memory) and
 // counts them per block.
+template <int ITEMS>
 __global__ void __launch_bounds__(kThreads) k_inv_flag(const unsigned long long* __restrict__ keys, int n,
                                                         unsigned char* __restrict__ flag,
                                                         int* __restrict__ block_sums)
 {
+    constexpr int kInvChunk = kThreads * ITEMS;
     __shared__ unsigned long long sk[kInvChunk + 2 * kWindow];
     const int base = blockIdx.x * kInvChunk;
     for (int j = threadIdx.x; j < kInvChunk + 2 * kWindow; j += kThreads) {
@@ -385,7 +436,7 @@ __global__ void __launch_bounds__(kThreads) k_inv_flag(const unsigned long long*
         return;
     }
     int c = 0;
-    for (int it = 0; it < kInvItems; ++it) {
+    for (int it = 0; it < ITEMS; ++it) {
         const int j = it * kThreads + threadIdx.x;
         const int i = base + j;
         if (i >= n)
@@ -447,6 +498,7 @@ __global__ void __launch_bounds__(1024) k_inv_scan(int* __restrict__ block_sums,
 }
 
 // Stable split into U (ukeys/uvals, in order) and F (fkeys/fvals, the first `cap` of them).
+template <int ITEMS>
 __global__ void __launch_bounds__(kThreads) k_inv_emit(const unsigned long long* __restrict__ keys,
                                                         const uint32_t* __restrict__ vals,
                                                         const unsigned char* __restrict__ flag, int n,
@@ -457,6 +509,7 @@ __global__ void __launch_bounds__(kThreads) k_inv_emit(const unsigned long long*
                                                         unsigned long long* __restrict__ fkeys,
                                                         uint32_t* __restrict__ fvals)
 {
+    constexpr int kInvChunk = kThreads * ITEMS;
     const int base = blockIdx.x * kInvChunk;
     const int fb0 = block_offsets[blockIdx.x];
     const int fb1 = blockIdx.x + 1 < gridDim.x ? block_offsets[blockIdx.x + 1] : ctl[0];
@@ -473,7 +526,7 @@ __global__ void __launch_bounds__(kThreads) k_inv_emit(const unsigned long long*
     if (threadIdx.x == 0)
         carry = block_offsets[blockIdx.x];
     __syncthreads();
-    for (int it = 0; it < kInvItems; ++it) {
+    for (int it = 0; it < ITEMS; ++it) {
         const int i = base + it * kThreads + threadIdx.x;
         const int f = i < n ? flag[i] : 0;
         const int x = warp_incl_scan(f);
@@ -502,46 +555,122 @@ __global__ void __launch_bounds__(kThreads) k_inv_emit(const unsigned long long*
     }
 }
 
-// ctl[1] |= 1 when U is not sorted.  Each thread checks a run of kVerifyRun consecutive keys
-// (16-byte loads) and the pair across the run's end.
-constexpr int kVerifyRun = 16;
+// ctl[1] |= 1 when U is not sorted.  A lane reads two neighbouring keys (a warp 512 consecutive bytes)
+// and takes the key after them from the next lane.  HBM-bound, 8 B a key: 69 us at
+// 16.7M (a run of 16 keys a thread, 128 bytes between the lanes of a load, took 200 to 228 us).
 __global__ void __launch_bounds__(kThreads) k_inv_verify(const unsigned long long* __restrict__ ukeys,
                                                           int n, int* __restrict__ ctl)
 {
     const long long m = n - ctl[0];
+    const int lane = threadIdx.x & 31;
+    const long long stride = 2LL * gridDim.x * kThreads;
     bool bad = false;
-    const long long stride = static_cast<long long>(gridDim.x) * kThreads * kVerifyRun;
-    for (long long s0 = (static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x) * kVerifyRun;
-         s0 + 1 < m; s0 += stride) {
-        if (s0 + kVerifyRun < m) {
-            const ulonglong2* p = reinterpret_cast<const ulonglong2*>(ukeys + s0);  // 128-byte aligned
-            unsigned long long prev = 0;
-#pragma unroll
-            for (int q = 0; q < kVerifyRun / 2; ++q) {
-                const ulonglong2 v = p[q];
-                bad = bad || (q > 0 && prev > v.x) || v.x > v.y;
-                prev = v.y;
-            }
-            bad = bad || prev > ukeys[s0 + kVerifyRun];
-        } else {
-            for (long long j = s0; j + 1 < m; ++j)
-                bad = bad || ukeys[j] > ukeys[j + 1];
-        }
+    // (the warp's first pair decides: all lanes stay for the shuffle)
+#pragma unroll 4
+    for (long long w0 = 2LL * (blockIdx.x * kThreads + threadIdx.x - lane); w0 < m; w0 += stride) {
+        const long long j = w0 + 2 * lane;
+        ulonglong2 v = make_ulonglong2(~0ull, ~0ull);
+        if (j + 1 < m)
+            v = *reinterpret_cast<const ulonglong2*>(ukeys + j);
+        else if (j < m)
+            v.x = ukeys[j];
+        unsigned long long after = __shfl_down_sync(kFullMask, v.x, 1);
+        if (lane == 31)
+            after = j + 2 < m ? ukeys[j + 2] : ~0ull;
+        bad = bad || v.x > v.y || v.y > after;
     }
-    if (__any_sync(kFullMask, bad) && (threadIdx.x & 31) == 0)
+    if (__any_sync(kFullMask, bad) && lane == 0)
         atomicOr(&ctl[1], 1);
 }
 
+// Sorts of a few thousand pairs by counting: a pair's place is the number of pairs before it, by key
+// and, for equal keys, by position (the stable order).  n^2 comparisons over all the SMs take less
+// than a radix sort's chain of nearly empty launches (4096 keys: 18 kernels, 105 us; this, with the
+// copy back, 11 us) and than a sort in one block (35 us: one SM's shared memory bounds it).
+// Each block holds all the keys in shared memory; a warp counts for kRankRows pairs at a time, its
+// lanes taking every 32nd key, so that one shared-memory read serves kRankRows comparisons.
+constexpr int kSmallSort = 8192;
+constexpr int kRankRows = 4;
+
+__device__ __forceinline__ void rank_sort(const unsigned long long* __restrict__ keys,
+                                          const uint32_t* __restrict__ vals, int n, unsigned long long* sk,
+                                          unsigned long long* __restrict__ out_keys, uint32_t* __restrict__ out_vals)
+{
+    const int lane = threadIdx.x & 31;
+    const int warps = gridDim.x * kWarps;
+    int i0 = (blockIdx.x * kWarps + (threadIdx.x >> 5)) * kRankRows;
+    if (blockIdx.x * kWarps * kRankRows >= n)
+        return;
+    for (int j = threadIdx.x; j < n; j += kThreads)
+        sk[j] = keys[j];
+    __syncthreads();
+    for (; i0 < n; i0 += warps * kRankRows) {
+        unsigned long long mine[kRankRows];
+        int before[kRankRows];
+#pragma unroll
+        for (int r = 0; r < kRankRows; ++r) {
+            mine[r] = sk[min(i0 + r, n - 1)];
+            before[r] = 0;
+        }
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) {
+            const unsigned long long k = sk[j];
+#pragma unroll
+            for (int r = 0; r < kRankRows; ++r)
+                before[r] += (k < mine[r] || (k == mine[r] && j < i0 + r)) ? 1 : 0;
+        }
+#pragma unroll
+        for (int r = 0; r < kRankRows; ++r) {
+            const int to = __reduce_add_sync(kFullMask, before[r]);
+            if (lane == r && i0 + r < n) {
+                out_keys[to] = mine[r];
+                out_vals[to] = vals[i0 + r];
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kThreads) k_small_sort(const unsigned long long* __restrict__ keys,
+                                                         const uint32_t* __restrict__ vals, int n,
+                                                         unsigned long long* __restrict__ out_keys,
+                                                         uint32_t* __restrict__ out_vals)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    rank_sort(keys, vals, n, reinterpret_cast<unsigned long long*>(smem_raw), out_keys, out_vals);
+}
+
+__global__ void k_copy_pairs(const unsigned long long* __restrict__ from_keys, const uint32_t* __restrict__ from_vals,
+                             int n, unsigned long long* __restrict__ keys, uint32_t* __restrict__ vals)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        keys[i] = from_keys[i];
+        vals[i] = from_vals[i];
+    }
+}
+
 // Picks the radix sort's job: the out-of-order pairs (fast path; ctl[3] = 0) or all pairs
-// (ctl[3] = n).  ctl[2] = the fast path's out-of-order count.
+// (ctl[3] = n).  ctl[2] = the fast path's out-of-order count.  Up to kSmallF out-of-order pairs go to
+// k_inv_rank and the radix sort gets an empty job, which its kernels leave at once.
+constexpr int kSmallF = 4096;
+__device__ __forceinline__ bool small_f(const int* ctl) { return ctl[3] == 0 && ctl[2] <= kSmallF; }
+
 __global__ void k_inv_mode(int n, int cap, int* __restrict__ ctl, SortJob* __restrict__ job,
                            SortJob fast_job, SortJob full_job)
 {
     const bool fast = ctl[1] == 0 && ctl[0] <= cap;
     ctl[2] = fast ? ctl[0] : 0;
     ctl[3] = fast ? 0 : n;
-    fast_job.n = ctl[0];
+    fast_job.n = ctl[0] <= kSmallF ? 0 : ctl[0];
     *job = fast ? fast_job : full_job;
+}
+
+// Few out-of-order pairs: sorted by counting into the alternate arrays, where the merge finds them.
+__global__ void __launch_bounds__(kThreads) k_inv_rank(const int* __restrict__ ctl, SortJob f)
+{
+    __shared__ unsigned long long sk[kSmallF];
+    if (!small_f(ctl))
+        return;
+    rank_sort(f.ka, f.va, ctl[2], sk, f.kb, f.vb);
 }
 
 // Entries of the sorted (k, v)[lo, hi) ordered before (key, val) by (key, value), plus lo.
@@ -565,14 +694,14 @@ __device__ __forceinline__ int rank_in(const unsigned long long* __restrict__ k,
 // bounds the F range that can fall inside it (usually empty).
 __global__ void __launch_bounds__(kThreads) k_inv_merge(const unsigned long long* __restrict__ ukeys,
                                                          const uint32_t* __restrict__ uvals,
-                                                         const unsigned long long* __restrict__ fkeys,
-                                                         const uint32_t* __restrict__ fvals, int n,
-                                                         const int* __restrict__ ctl,
+                                                         SortJob f, int n, const int* __restrict__ ctl,
                                                          unsigned long long* __restrict__ keys,
                                                          uint32_t* __restrict__ vals)
 {
     if (ctl[3] != 0)
         return;  // the full sort ran
+    const unsigned long long* __restrict__ fkeys = small_f(ctl) ? f.kb : f.ka;
+    const uint32_t* __restrict__ fvals = small_f(ctl) ? f.vb : f.va;
     const int nf = ctl[2], m = n - nf;
     const int useg = (m + kMergeSeg - 1) / kMergeSeg;
     const int fseg = (nf + kThreads - 1) / kThreads;
@@ -610,7 +739,15 @@ __global__ void __launch_bounds__(kThreads) k_inv_merge(const unsigned long long
 
 } // namespace
 
-int adaptive_sort_blocks(int n) { return n > 0 ? (n + kInvChunk - 1) / kInvChunk : 1; }
+int adaptive_sort_blocks(int n)
+{
+    // the largest block count of any n' <= n: a workspace serves every smaller system
+    const int m = n < kInvSmall ? n : kInvSmall - 1;
+    const int few = (m + kThreads * kInvItemsSmall - 1) / (kThreads * kInvItemsSmall);
+    const int many = (n + kThreads * kInvItems - 1) / (kThreads * kInvItems);
+    const int b = few > many ? few : many;
+    return b > 0 ? b : 1;
+}
 int adaptive_sort_cap(int n) { return n / 8 > 4096 ? n / 8 : 4096; }
 
 void launch_radix_sort_adaptive(unsigned long long* keys, uint32_t* vals, int n, int bits,
@@ -622,24 +759,48 @@ void launch_radix_sort_adaptive(unsigned long long* keys, uint32_t* vals, int n,
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int blocks = adaptive_sort_blocks(n);
+    if (n <= kSmallSort && bits == 64) {
+        static std::atomic<bool> attr_set[kMaxDevices];
+        if (dev < 0 || dev >= kMaxDevices || !attr_set[dev].load()) {
+            cudaFuncSetAttribute(k_small_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSort * 8);
+            if (dev >= 0 && dev < kMaxDevices)
+                attr_set[dev].store(true);
+        }
+        const int rows = kWarps * kRankRows;
+        count_launch(2);
+        k_small_sort<<<(n + rows - 1) / rows, kThreads, static_cast<size_t>(n) * 8, s>>>(keys, vals, n, ws.keys_alt,
+                                                                                         ws.vals_alt);
+        k_copy_pairs<<<(n + 255) / 256, 256, 0, s>>>(ws.keys_alt, ws.vals_alt, n, keys, vals);
+        return;
+    }
+    const int items = inv_items(n);
+    const int blocks = (n + kThreads * items - 1) / (kThreads * items);
     count_launch(3);
-    k_inv_flag<<<blocks, kThreads, 0, s>>>(keys, n, aws.flag, aws.block_sums);
+    if (items == kInvItems)
+        k_inv_flag<kInvItems><<<blocks, kThreads, 0, s>>>(keys, n, aws.flag, aws.block_sums);
+    else
+        k_inv_flag<kInvItemsSmall><<<blocks, kThreads, 0, s>>>(keys, n, aws.flag, aws.block_sums);
     k_inv_scan<<<1, 1024, 0, s>>>(aws.block_sums, blocks, aws.ctl);
-    k_inv_emit<<<blocks, kThreads, 0, s>>>(keys, vals, aws.flag, n, aws.block_sums, aws.cap,
-                                           aws.ctl, ws.keys_alt, ws.vals_alt, aws.fkeys, aws.fvals);
-    int vb = (n + kThreads - 1) / kThreads;
-    vb = vb < 4 * sms ? vb : 4 * sms;
+    if (items == kInvItems)
+        k_inv_emit<kInvItems><<<blocks, kThreads, 0, s>>>(keys, vals, aws.flag, n, aws.block_sums, aws.cap, aws.ctl,
+                                                          ws.keys_alt, ws.vals_alt, aws.fkeys, aws.fvals);
+    else
+        k_inv_emit<kInvItemsSmall><<<blocks, kThreads, 0, s>>>(keys, vals, aws.flag, n, aws.block_sums, aws.cap,
+                                                               aws.ctl, ws.keys_alt, ws.vals_alt, aws.fkeys,
+                                                               aws.fvals);
+    int vb = (n / 2 + kThreads - 1) / kThreads;
+    vb = vb < 8 * sms ? vb : 8 * sms;
     count_launch(2);
     k_inv_verify<<<vb, kThreads, 0, s>>>(ws.keys_alt, n, aws.ctl);
     const SortJob fast_job{aws.fkeys, aws.fvals, aws.falt_keys, aws.falt_vals, 0};
     const SortJob full_job{keys, vals, ws.keys_alt, ws.vals_alt, n};
     k_inv_mode<<<1, 1, 0, s>>>(n, aws.cap, aws.ctl, aws.job, fast_job, full_job);
+    count_launch();
+    k_inv_rank<<<kSmallF / (kWarps * kRankRows), kThreads, 0, s>>>(aws.ctl, fast_job);
     // one radix sort: of F in place on the fast path, else of all of (keys, vals)
     enqueue_sort(keys, vals, n, bits, ws, err, s, aws.job);
     count_launch();
-    k_inv_merge<<<8 * sms, kThreads, 0, s>>>(ws.keys_alt, ws.vals_alt, aws.fkeys, aws.fvals, n,
-                                             aws.ctl, keys, vals);
+    k_inv_merge<<<8 * sms, kThreads, 0, s>>>(ws.keys_alt, ws.vals_alt, fast_job, n, aws.ctl, keys, vals);
 }
 
 } // namespace bz
