@@ -23,6 +23,8 @@
 #include "bz_common.cuh"
 #include "bz_kernels.h"
 
+#include <cuda_fp16.h>
+
 namespace bz {
 
 namespace {
@@ -33,6 +35,7 @@ constexpr int kSpill = 8192;      // per-warp global spill area (oldest entries)
 constexpr int kList = 64;         // leaf list
 constexpr int kNodes = 128;       // accepted nodes evaluated per flush
 constexpr int kTile = 128;
+constexpr int kMaskPitch = 40;  // a target's word q lies 8 banks past its word q - 1
 constexpr int kFlushParticles = 256;  // listed leaf particles that trigger a flush
 constexpr int kIndexBits = 26;
 constexpr int kIndexMask = (1 << kIndexBits) - 1;
@@ -45,7 +48,8 @@ template <bool QUAD> struct __align__(16) WarpSmem {
     union {
         struct {
             float4 tile[kTile];
-            unsigned mask[kTile / 32][32];  // per-lane in-cutoff bits of the tile
+            unsigned mask[kTile / 32][kMaskPitch];  // per-lane in-cutoff bits of the tile
+            uint4 brow[QUAD ? 1 : kTile / 2];  // cutoff filter: FP16 rows of half a tile's sources
         };
         struct {
             // accepted nodes, two to an entry so that packed FP32 instructions take both:
@@ -54,6 +58,8 @@ template <bool QUAD> struct __align__(16) WarpSmem {
             float2 nd_tr[QUAD ? kNodes / 2 : 1];  // tr(Q) eps^2 (Newtonian) or -tr(Q) / 2 (split)
         };
     };
+    uint4 arow[QUAD ? 1 : 32];  // cutoff filter: FP16 rows of the targets
+    float4 frame;     // ... centre of the group, scale (0: too wide for FP16, scalar filter)
     float4 tgt[32];   // the group's targets (slots past its size repeat the first)
     int tidx[kTile];  // sorted index of each tile source (pairs recorded, potentials)
     unsigned stack[kStack];  // opened nodes: first child | (children - 1) << kIndexBits
@@ -615,6 +621,118 @@ __device__ __forceinline__ void flush_nodes(WarpSmem<QUAD>& w, int m, const Tree
     __syncwarp();
 }
 
+// ---- cutoff filter on the tensor cores -----------------------------------------------------
+// Which of a tile's 128 sources lie inside each of the 32 targets' cutoff spheres: the signs of
+//   D = |s|^2 - 2 s t + |t|^2 - r^2 = [-2t, 1, 1, Thi, Tlo] . [s, Shi, Slo, 1, 1],
+// a 32 x 128 x 8 product (mma m16n8k8, FP16 operands, FP32 sums), s and t in units of r_cut / 8
+// from the group's centre.  S = |s|^2 of the ROUNDED s and T = |t|^2 - r^2 are split into two FP16
+// parts, so D is the exact distance test of the rounded points up to 2^-22 of S and T; r carries
+// the rounding of both points.  The marked set therefore contains every pair inside the cutoff
+// (and about 0.5 % more), and the pair law's own FP32 test decides the rest, so the sums are those
+// of the scalar filter, which spends nine instructions on each listed pair (4.0 to 6.7 listed for
+// each evaluated one): MEASURED
+constexpr float kFilterScale = 8.0f;
+constexpr float kFilterMaxExtent = 64.0f;  // of the group's half box, scaled: T and S stay far below 65504
+
+__device__ __forceinline__ unsigned pack_h2(float a, float b)
+{
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const unsigned*>(&h);
+}
+
+// One FP16 row: {x, y, z, hi, lo, one, one, 0} of the point x, y, z; returns the rounded point's
+// square norm through n2.
+__device__ __forceinline__ float round_point(float& x, float& y, float& z)
+{
+    x = __half2float(__float2half_rn(x));
+    y = __half2float(__float2half_rn(y));
+    z = __half2float(__float2half_rn(z));
+    return fmaf(x, x, fmaf(y, y, z * z));
+}
+
+template <class W>
+__device__ __forceinline__ void filter_group(W& w, const float4 me, const float* gc, const float* ghalf, float rcut)
+{
+    const int lane = threadIdx.x & 31;
+    const float sc = kFilterScale / rcut;
+    const float ext = fmaxf(ghalf[0], fmaxf(ghalf[1], ghalf[2])) * sc;
+    // position errors in scaled units: FP16 rounding of both points (sqrt(3) 2^-11 of their
+    // coordinates, at most ext and ext + 8), FP32 rounding of the subtraction
+    const float far = fmaxf(fabsf(gc[0]), fmaxf(fabsf(gc[1]), fabsf(gc[2])));
+    const float d = 0.001f * (2.0f * ext + kFilterScale) + 1.0e-6f * sc * far;
+    const float r = kFilterScale + d;
+    const float r2 = r * r + 1.2e-5f * (2.0f * ext + kFilterScale) * (2.0f * ext + kFilterScale);
+    float x = (me.x - gc[0]) * sc, y = (me.y - gc[1]) * sc, z = (me.z - gc[2]) * sc;
+    const float t = round_point(x, y, z) - r2;
+    const float hi = __half2float(__float2half_rn(t));
+    w.arow[lane] = make_uint4(pack_h2(-2.0f * x, -2.0f * y), pack_h2(-2.0f * z, 1.0f), pack_h2(1.0f, hi),
+                              pack_h2(t - hi, 0.0f));
+    // (a NaN or infinite extent fails the comparison too)
+    if (lane == 0)
+        w.frame = make_float4(gc[0], gc[1], gc[2], ext <= kFilterMaxExtent && d < kFilterScale ? sc : 0.0f);
+}
+
+// Fills w.mask for the nb sources of the tile: bit b of word q of target j is source 32 q + b.
+template <class W> __device__ __forceinline__ void filter_tile(W& w, int nb, const float4 frame)
+{
+    const int lane = threadIdx.x & 31;
+    const int row = lane >> 2, q = lane & 3;
+    const unsigned* ar = reinterpret_cast<const unsigned*>(w.arow);
+    unsigned a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        a[i] = ar[(row + 8 * i) * 4 + q];
+    unsigned m[4] = {0u, 0u, 0u, 0u};
+    const uint32_t bbase = smem_u32(w.brow) + lane * 16;
+#pragma unroll 1
+    for (int h = 1; h >= 0; --h) {
+        // column n of n-tile t of this half is source 32 (n / 2) + 16 h + 2 t + n % 2
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int rr = lane + 32 * u, n = rr & 7;
+            const int j = 32 * (n >> 1) + 16 * h + 2 * (rr >> 3) + (n & 1);
+            uint4 v = make_uint4(0u, pack_h2(0.0f, 30000.0f), 0u, 0u);  // past the end: never inside
+            if (j < nb) {
+                const float4 s4 = w.tile[j];
+                float x = (s4.x - frame.x) * frame.w, y = (s4.y - frame.y) * frame.w, z = (s4.z - frame.z) * frame.w;
+                const float s2 = round_point(x, y, z);
+                const float hi = __half2float(__float2half_rn(s2));
+                v = make_uint4(pack_h2(x, y), pack_h2(z, hi), pack_h2(s2 - hi, 1.0f), pack_h2(1.0f, 0.0f));
+            }
+            w.brow[rr] = v;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int g = 1; g >= 0; --g) {
+            unsigned b[4];
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                         : "r"(bbase + g * 512)
+                         : "memory");
+#pragma unroll
+            for (int t = 3; t >= 0; --t) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float c[4];
+                    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+                        "{%7, %7, %7, %7};"
+                        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                        : "r"(a[2 * i]), "r"(a[2 * i + 1]), "r"(b[t]), "f"(0.0f));
+                    m[2 * i] = __funnelshift_l(__float_as_uint(c[1]), m[2 * i], 1);
+                    m[2 * i] = __funnelshift_l(__float_as_uint(c[0]), m[2 * i], 1);
+                    m[2 * i + 1] = __funnelshift_l(__float_as_uint(c[3]), m[2 * i + 1], 1);
+                    m[2 * i + 1] = __funnelshift_l(__float_as_uint(c[2]), m[2 * i + 1], 1);
+                }
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        w.mask[q][row + 8 * i] = m[i];
+    __syncwarp();
+}
+
 template <bool PERIODIC, bool SPLIT, bool POT, bool SLICED, class W>
 __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure, const float4* __restrict__ pos4,
                                              const TreeArrays& t, const WalkParams& p,
@@ -843,7 +961,12 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
             // r2 <= rcut2 exactly when r2 - next_float(rcut2) is negative (a float difference
             // has the exact sign), so the sign bit is the mask bit: one funnel shift appends it
             const float rc2n = __uint_as_float(__float_as_uint(p.rcut2) + 1u);
-            for (int wd = 0; wd < nw; ++wd) {
+            // the walks that only filter mark on the tensor cores; then a marked pair takes the
+            // pair law's own distance test
+            const float4 frame = SLICED ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : w.frame;
+            if (!SLICED && frame.w > 0.0f)
+                filter_tile(w, nb, frame);
+            for (int wd = 0; frame.w == 0.0f && wd < nw; ++wd) {
                 const int qb = wd << 5;
                 unsigned m = 0u;
                 if (qb + 32 <= nb) {
@@ -865,7 +988,6 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
                     }
                 }
                 w.mask[wd][lane] = m;
-                evald += __popc(m);
             }
             int wd = 0;
             unsigned m = w.mask[0][lane];
@@ -877,7 +999,7 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
                 const int b = __ffs(m) - 1;
                 m &= m - 1u;
                 const float4 s4 = w.tile[(wd << 5) + b];
-                pair_fast<SPLIT>(s4, tx, ty, tz, p.eps2, p.rcut2, false, sk, fx, fy, fz);
+                evald += pair_fast<SPLIT>(s4, tx, ty, tz, p.eps2, p.rcut2, !SLICED, sk, fx, fy, fz);
                 if (rec)
                     record(s4, w.tidx[(wd << 5) + b]);
             }
@@ -1015,6 +1137,8 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
             ghalf[a] = __fmul_rn(0.5f, __fsub_rn(gmax[a], gmin[a]));
         }
 
+        if (!SLICED && cut)
+            filter_group(w, me, gc, ghalf, rcut);
         // With a cutoff, leaves wholly inside it for every target ("sure": the farthest corners of
         // leaf and group) are listed from the far end of the leaf list and summed without the
         // per-lane filter; the margin covers the rounding of a pair's own distance test.
