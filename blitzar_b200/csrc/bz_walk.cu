@@ -1099,6 +1099,8 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
     fence_mbar_init();
     __syncwarp();
     constexpr bool SLICED = walk_sliced<SPLIT, QUAD>();
+    // (adaptive steps: force-only walks of the octree solver)
+    const bool adaptive = !PERIODIC && !SPLIT && !POT && p.active != nullptr;
     const bool cut = p.rcut2 > 0.0f;
     const float inv2rs = SPLIT ? 0.5f / p.rsplit : 0.0f;
     const float rcut = __fsqrt_rn(p.rcut2);
@@ -1114,16 +1116,33 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
         if (g >= ngroups)
             break;
         const int g0 = gstart[g];
-        const int gn = gstart[g + 1] - g0;
-        const int ti = g0 + lane;
+        const int members = gstart[g + 1] - g0;
+        const float4 member = pos4[lane < members ? g0 + lane : g0];
+        // The targets this warp evaluates, one owner lane each: the group's members or, in
+        // adaptive substeps, those of them that close their step (a group without one is not
+        // walked).  Boxes and decisions are the whole group's either way.  (96 clusters, six levels:
+        // MEASURED a substep.)
+        int gn = members, ti = g0 + lane;
+        float4 me = member;
+        if (adaptive) {
+            const unsigned closing = __ballot_sync(kFullMask, lane < members && p.active[g0 + lane] != 0);
+            if (closing == 0u)
+                continue;
+            gn = __popc(closing);
+            unsigned m = closing;
+            for (int skip = lane < gn ? lane : 0; skip > 0; --skip)
+                m &= m - 1u;
+            const int src = __ffs(m) - 1;  // the closing member of this lane's rank
+            ti = g0 + src;
+            me.x = __shfl_sync(kFullMask, member.x, src);
+            me.y = __shfl_sync(kFullMask, member.y, src);
+            me.z = __shfl_sync(kFullMask, member.z, src);
+            me.w = __shfl_sync(kFullMask, member.w, src);
+        }
         const bool valid = lane < gn;
-        const float4 me = pos4[valid ? ti : g0];
-        // adaptive steps: only groups holding a target that closes its step are walked
-        if (p.active != nullptr && !__any_sync(kFullMask, valid && p.active[ti] != 0))
-            continue;
         const LaneMap lanes(gn, SLICED);
         w.tgt[lane] = me;
-        float gmin[3] = {me.x, me.y, me.z}, gmax[3] = {me.x, me.y, me.z};
+        float gmin[3] = {member.x, member.y, member.z}, gmax[3] = {member.x, member.y, member.z};
 #pragma unroll
         for (int a = 0; a < 3; ++a)
             for (int off = 16; off > 0; off >>= 1) {
@@ -1361,14 +1380,16 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
                     raise_error(err, kErrListCapacity);
             }
         }
-        const unsigned long long ev = __reduce_add_sync(kFullMask, valid ? evald : 0u);
+        unsigned long long ev = __reduce_add_sync(kFullMask, valid ? evald : 0u);
+        if (adaptive)  // (the counters report the walked groups' members)
+            ev = static_cast<unsigned long long>(cnt_pp) * members;
         if (lane == 0) {
             if (o.n_pp)
                 o.n_pp[g] = cnt_pp;
             if (o.n_pn)
                 o.n_pn[g] = cnt_pn;
             if (o.totals) {
-                const unsigned long long ng = static_cast<unsigned long long>(gn);
+                const unsigned long long ng = static_cast<unsigned long long>(members);
                 atomicAdd(&o.totals[0], ng * cnt_pp);
                 atomicAdd(&o.totals[1], ng * cnt_pn);
                 atomicAdd(&o.totals[2], ev);
