@@ -317,9 +317,11 @@ __device__ __forceinline__ void pair_pn(const float4 mo, const float4 qa, const 
 // and trm = -tr(Q) eps^2/3, algebraically the same as the traceful form (the m/s^3 + (15/2 dQd/s^7 -
 // 3/2 tr/s^5)) d - 3 Qd/s^5 of pair_pn).  Used only when eps^2 exceeds the minimum distance^2,
 // so the minimum-distance guard of pair_pn can never trigger.
+// The potential's expansion collapses the same way: -m/s - 3/2 (dQ'd + trm)/s^5, negated in np.
 // nx, ny, nz: the target's negated position; q = -3 Q' (xx xy xz yy yz zz), trm scaled by -3 too.
+template <bool POT>
 __device__ __forceinline__ void pair_pn_newton2(F2 x, F2 y, F2 z, F2 m, const F2* q, F2 trm, F2 nx,
-                                                F2 ny, F2 nz, F2 eps2, F2& fx, F2& fy, F2& fz)
+                                                F2 ny, F2 nz, F2 eps2, F2& fx, F2& fy, F2& fz, F2& np)
 {
     const F2 dx = add2(x, nx), dy = add2(y, ny), dz = add2(z, nz);
     const F2 rinv = rsqrt2(fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, eps2))));
@@ -334,6 +336,8 @@ __device__ __forceinline__ void pair_pn_newton2(F2 x, F2 y, F2 z, F2 m, const F2
     fx = fma2(c0, dx, fma2(t5, qx, fx));
     fy = fma2(c0, dy, fma2(t5, qy, fy));
     fz = fma2(c0, dz, fma2(t5, qz, fz));
+    if (POT)
+        np = fma2(m, rinv, fma2(mul2(t5, f2(-0.5f)), dqd, np));
 }
 
 // Force-only quadrupole interaction with the split kernel of two nodes at a time, softening above
@@ -375,10 +379,11 @@ __device__ __forceinline__ void pair_pn_split2(F2 x, F2 y, F2 z, F2 m, const F2*
     fz = fma2(c0, dz, fma2(c2, qz, fz));
 }
 
-// As pair_fast without a cutoff, for two sources at a time.
-template <bool SPLIT>
-__device__ __forceinline__ void pair_fast2(F2 x, F2 y, F2 z, F2 m, F2 nx, F2 ny, F2 nz, F2 eps2,
-                                           const SplitK& k, F2& fx, F2& fy, F2& fz)
+// As pair_fast without a cutoff, for two sources at a time; POT: np collects mp / s, mp the masses
+// that count for the potential (not the target's own).
+template <bool SPLIT, bool POT>
+__device__ __forceinline__ void pair_fast2(F2 x, F2 y, F2 z, F2 m, F2 mp, F2 nx, F2 ny, F2 nz, F2 eps2,
+                                           const SplitK& k, F2& fx, F2& fy, F2& fz, F2& np)
 {
     const F2 dx = add2(x, nx), dy = add2(y, ny), dz = add2(z, nz);
     const F2 s2 = add2(fma2(dx, dx, fma2(dy, dy, mul2(dz, dz))), eps2);
@@ -401,6 +406,8 @@ __device__ __forceinline__ void pair_fast2(F2 x, F2 y, F2 z, F2 m, F2 nx, F2 ny,
     fx = fma2(f, dx, fx);
     fy = fma2(f, dy, fy);
     fz = fma2(f, dz, fz);
+    if (POT)
+        np = fma2(mp, rinv, np);
 }
 
 struct Acc {
@@ -499,9 +506,9 @@ __device__ __forceinline__ void flush_nodes(WarpSmem<QUAD>& w, int m, const Tree
                                             Acc& acc)
 {
     const int lane = threadIdx.x & 31;
-    // force-only quadrupoles with eps^2 > min distance^2 are evaluated two nodes at a time; the
-    // Newtonian ones in the traceless form
-    const bool packed = QUAD && !POT && p.eps2 > p.min_dist2;
+    // quadrupoles with eps^2 > min distance^2 are evaluated two nodes at a time (with the split
+    // kernel, forces only); the Newtonian ones in the traceless form
+    const bool packed = QUAD && !(POT && SPLIT) && p.eps2 > p.min_dist2;
     const int pairs = (m + 1) >> 1;
     if ((m & 1) && lane == 0)
         w.nlist[m] = w.nlist[m - 1];  // an odd list's last node is paired with itself, massless
@@ -563,14 +570,14 @@ __device__ __forceinline__ void flush_nodes(WarpSmem<QUAD>& w, int m, const Tree
         rows.load(w, lm, row0);
         float none = 0.0f;
         if (packed) {
-            F2 nx[R], ny[R], nz[R], fx[R], fy[R], fz[R];
+            F2 nx[R], ny[R], nz[R], fx[R], fy[R], fz[R], np[R];
             const F2 eps2 = f2(p.eps2);
 #pragma unroll
             for (int k = 0; k < R; ++k) {
                 nx[k] = f2(-rows.tx[k]);
                 ny[k] = f2(-rows.ty[k]);
                 nz[k] = f2(-rows.tz[k]);
-                fx[k] = fy[k] = fz[k] = f2(0.0f);
+                fx[k] = fy[k] = fz[k] = np[k] = f2(0.0f);
             }
 #pragma unroll 1
             for (int j = lm.slice; j < pairs; j += lm.nslices) {
@@ -585,8 +592,8 @@ __device__ __forceinline__ void flush_nodes(WarpSmem<QUAD>& w, int m, const Tree
                         pair_pn_split2({a.x}, {a.y}, {b.x}, {b.y}, q, tr, nx[k], ny[k], nz[k], eps2, inv2rs,
                                        fx[k], fy[k], fz[k]);
                     else
-                        pair_pn_newton2({a.x}, {a.y}, {b.x}, {b.y}, q, tr, nx[k], ny[k], nz[k], eps2, fx[k],
-                                        fy[k], fz[k]);
+                        pair_pn_newton2<POT>({a.x}, {a.y}, {b.x}, {b.y}, q, tr, nx[k], ny[k], nz[k], eps2, fx[k],
+                                             fy[k], fz[k], np[k]);
                 }
             }
 #pragma unroll
@@ -594,6 +601,8 @@ __device__ __forceinline__ void flush_nodes(WarpSmem<QUAD>& w, int m, const Tree
                 rows.f[0][k] = lo(fx[k]) + hi(fx[k]);
                 rows.f[1][k] = lo(fy[k]) + hi(fy[k]);
                 rows.f[2][k] = lo(fz[k]) + hi(fz[k]);
+                if (POT)
+                    rows.f[POT ? 3 : 0][k] = -(lo(np[k]) + hi(np[k]));
             }
         } else {
 #pragma unroll 1
@@ -898,9 +907,13 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
             // filled up with massless sources to whole pairs for every slice)
             evald += nb;
             const int npad = (nb + 2 * lm.nslices - 1) & ~(2 * lm.nslices - 1);
-            if (SLICED && fast) {
-                for (int j = nb + lane; j < npad; j += 32)
+            const bool packed = SLICED && !cut && !(POT && SPLIT) && p.eps2 > p.min_dist2;
+            if (packed) {
+                for (int j = nb + lane; j < npad; j += 32) {
                     w.tile[j] = make_float4(tx, ty, tz, 0.0f);
+                    if (POT)
+                        w.tidx[j] = -1;
+                }
                 __syncwarp();
             }
             for_rows<SLICED>(lm, [&](auto rc, int row0) {
@@ -908,32 +921,39 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
                 Rows<R, POT ? 4 : 3> rows;
                 rows.load(w, lm, row0);
                 float none = 0.0f;
-                if (SLICED && fast) {
-                    F2 nx[R], ny[R], nz[R], fx[R], fy[R], fz[R];
+                const int t0 = self_index - lane + lm.slot + kSlots * row0;
+                if (packed) {
+                    F2 nx[R], ny[R], nz[R], fx[R], fy[R], fz[R], np[R];
                     const F2 eps2 = f2(p.eps2);
 #pragma unroll
                     for (int k = 0; k < R; ++k) {
                         nx[k] = f2(-rows.tx[k]);
                         ny[k] = f2(-rows.ty[k]);
                         nz[k] = f2(-rows.tz[k]);
-                        fx[k] = fy[k] = fz[k] = f2(0.0f);
+                        fx[k] = fy[k] = fz[k] = np[k] = f2(0.0f);
                     }
 #pragma unroll 1
                     for (int j = lm.slice; j < npad; j += 2 * lm.nslices) {
                         const float4 s0 = w.tile[j], s1 = w.tile[j + lm.nslices];
+                        const int i0 = POT ? w.tidx[j] : 0, i1 = POT ? w.tidx[j + lm.nslices] : 0;
                         const F2 x = f2(s0.x, s1.x), y = f2(s0.y, s1.y), z = f2(s0.z, s1.z), m = f2(s0.w, s1.w);
 #pragma unroll
-                        for (int k = 0; k < R; ++k)
-                            pair_fast2<SPLIT>(x, y, z, m, nx[k], ny[k], nz[k], eps2, sk, fx[k], fy[k], fz[k]);
+                        for (int k = 0; k < R; ++k) {
+                            const int own = t0 + kSlots * k;
+                            const F2 mp = POT ? f2(i0 == own ? 0.0f : s0.w, i1 == own ? 0.0f : s1.w) : m;
+                            pair_fast2<SPLIT, POT>(x, y, z, m, mp, nx[k], ny[k], nz[k], eps2, sk, fx[k], fy[k], fz[k],
+                                                   np[k]);
+                        }
                     }
 #pragma unroll
                     for (int k = 0; k < R; ++k) {
                         rows.f[0][k] = lo(fx[k]) + hi(fx[k]);
                         rows.f[1][k] = lo(fy[k]) + hi(fy[k]);
                         rows.f[2][k] = lo(fz[k]) + hi(fz[k]);
+                        if (POT)
+                            rows.f[POT ? 3 : 0][k] = -(lo(np[k]) + hi(np[k]));
                     }
                 } else {
-                    const int t0 = self_index - lane + lm.slot + kSlots * row0;
 #pragma unroll 1
                     for (int j = lm.slice; j < nb; j += lm.nslices) {
                         const float4 s4 = w.tile[j];
