@@ -131,6 +131,7 @@ struct bz_handle {
         bool enabled = false;
         int* pair_src = nullptr;  // [capacity * kPairSlots]
         int* pair_cnt = nullptr;  // [capacity]
+        uint4* feat = nullptr;    // [capacity] offset features of the current positions
     } learn;
 };
 
@@ -326,7 +327,7 @@ void enqueue_forces(bz_handle* h, bool kick, bool want_pot, bool mesh_forked = f
         const float hcell = static_cast<float>(h->cfg.box_length / h->cfg.treepm_grid_size);
         launch_mlp_pairs(h->learn.params, d.pos4, n, h->learn.pair_src, h->learn.pair_cnt, hcell,
                          static_cast<float>(h->cfg.box_length), h->learn.scale, d.acc[0], d.acc[1],
-                         d.acc[2], d.err, h->stream);
+                         d.acc[2], d.err, h->stream, h->learn.feat);
     }
     record(h, kPhIntegrate);
     if (kick) {
@@ -1834,7 +1835,7 @@ bool learn_pairs_alloc(bz_handle* h)
     if (L.pair_src)
         return true;
     return dalloc(h, &L.pair_src, h->capacity * static_cast<size_t>(kPairSlots)) &&
-           dalloc(h, &L.pair_cnt, h->capacity);
+           dalloc(h, &L.pair_cnt, h->capacity) && dalloc(h, &L.feat, h->capacity);
 }
 
 void drop_graphs(bz_handle* h)

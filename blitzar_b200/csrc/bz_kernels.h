@@ -309,7 +309,7 @@ void launch_mlp_forward(const float* params, const float* in6, int n, float scal
                         int* err, cudaStream_t s);
 void launch_mlp_pairs(const float* params, const float4* pos4, int n, const int* pair_src,
                       const int* pair_cnt, float h, float box, float scale, float* ax, float* ay,
-                      float* az, int* err, cudaStream_t s);
+                      float* az, int* err, cudaStream_t s, uint4* feat);
 
 // ---------------------------------------------------------------- diagnostics (bz_diag.cu)
 // FP64 reference accelerations for the listed (sorted-order) targets: direct sum (open) or

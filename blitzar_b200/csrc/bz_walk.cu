@@ -1142,7 +1142,7 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
         const float4 member = pos4[lane < members ? g0 + lane : g0];
         // The targets this warp evaluates, one owner lane each: the group's members or, in
         // adaptive substeps, those of them that close their step (a group without one is not
-        // walked).  Boxes and decisions are the whole group's either way.  (96 clusters, six levels:
+        // walked).  Boxes and decisions are the whole group's either way.  (96 clusters, six levels, a
         // block of 32 substeps: walks 19.6 -> 16.9 ms.)
         int gn = members, ti = g0 + lane;
         float4 me = member;
