@@ -283,7 +283,8 @@ void enqueue_forces(bz_handle* h, bool kick, bool want_pot, bool mesh_forked = f
     const int root_level = h->systems > 0 ? kSystemLevels : 0;
     launch_tree_build(d.keys, d.pos4, n, h->cfg.leaf_capacity, h->tree, d.err,
                       h->stream, root_level, h->cfg.multipole_order >= 2);
-    launch_groups(h->tree, n, h->cfg.walk_group_size, root_level, d.keys, h->groups, h->stream);
+    launch_groups(h->tree, n, h->cfg.walk_group_size, root_level, d.keys, h->groups,
+                  !periodic(h), h->stream);
     record(h, kPhMesh);
     if (h->cfg.solver == BZ_SOLVER_TREEPM && h->pm && !overlap) {
         pm_forces(h->pm, d.pos4, n, d.acc[0], d.acc[1], d.acc[2], h->stream);
@@ -717,6 +718,7 @@ bz_status bz_create(const bz_config* cfg, size_t capacity, bz_handle** out)
     GroupTable& gt = h->groups;
     ok = ok && dalloc(h, &gt.flag, group_flag_bytes(static_cast<int>(n))) && dalloc(h, &gt.gstart, n + 1) && dalloc(h, &gt.ngroups, 1) &&
          dalloc(h, &gt.groot, n + 1) && dalloc(h, &gt.sysroot, kMaxSystems) &&
+         dalloc(h, &gt.order, kOrderGroups) && dalloc(h, &gt.ordered, 1) &&
          (cfg->adaptive_max_level == 0 ||
           (dalloc(h, &h->ad.st.level, n) && dalloc(h, &h->ad.st.ax, n) && dalloc(h, &h->ad.st.ay, n) &&
            dalloc(h, &h->ad.st.az, n) && dalloc(h, &h->ad.st.updates, 1) && dalloc(h, &h->ad.active, n) &&
@@ -732,6 +734,7 @@ bz_status bz_create(const bz_config* cfg, size_t capacity, bz_handle** out)
     cudaMemsetAsync(sw.state, 0, words * sizeof(unsigned long long), h->stream);
     cudaMemsetAsync(sw.epoch, 0, sizeof(uint32_t), h->stream);
     cudaMemsetAsync(d.err, 0, sizeof(int), h->stream);
+    cudaMemsetAsync(gt.ordered, 0, sizeof(int), h->stream);
     if (cfg->solver == BZ_SOLVER_TREEPM) {
         int perr = 0;
         if (isolated(h)) {
@@ -1527,7 +1530,7 @@ bz_status adaptive_steps(bz_handle* h, double dt, uint32_t nsteps)
                 launch_tree_build(d.keys, d.pos4, n, h->cfg.leaf_capacity, h->tree, d.err,
                                   h->stream, root_level, h->cfg.multipole_order >= 2);
                 launch_groups(h->tree, n, h->cfg.walk_group_size, root_level, d.keys, h->groups,
-                              h->stream);
+                              !periodic(h), h->stream);
             } else {
                 double* const* st = d.st[h->cur];
                 record(h, kPhKeys);

@@ -231,6 +231,50 @@ __global__ void __launch_bounds__(kThreads) k_flag_emit(const unsigned char* __r
         gstart[*ngroups] = n;
 }
 
+// slot[s]++, one atomic for the lanes of a warp that share s.
+__device__ __forceinline__ int take_slot(int* slot, int s)
+{
+    const unsigned peers = __match_any_sync(__activemask(), s);
+    const int leader = __ffs(peers) - 1;
+    int at = 0;
+    if ((threadIdx.x & 31) == leader)
+        at = atomicAdd(&slot[s], __popc(peers));
+    return __shfl_sync(peers, at, leader) + __popc(peers & lanemask_lt());
+}
+
+// The order in which the walk takes the groups of a small system: by falling size (a counting sort
+// over the sizes in one block; equal sizes in any order, which no result depends on).  A walk of a
+// few groups a warp ends when its last long group does, so the long ones go first (Plummer 65k,
+// 3700 groups: 0.395 -> 0.35 ms; 200k with potentials, 11 thousand: 1.20 -> 1.09 ms).  With at most one
+// group a warp, or with more than kOrderGroups (many a warp: the tail is short), the order is not
+// used; nor for periodic boxes, whose groups are cut from a nearly uniform lattice.
+__global__ void __launch_bounds__(1024) k_group_order(const int* __restrict__ gstart, const int* __restrict__ ngroups_ptr,
+                                                      int warps, int* __restrict__ order, int* __restrict__ ordered)
+{
+    const int ng = *ngroups_ptr;
+    const bool use = ng > warps && ng <= kOrderGroups;
+    if (threadIdx.x == 0)
+        *ordered = use ? 1 : 0;
+    if (!use)
+        return;
+    __shared__ int slot[kGroupMax];  // slot[s]: groups of kGroupMax - s targets, then their next place
+    if (threadIdx.x < kGroupMax)
+        slot[threadIdx.x] = 0;
+    __syncthreads();
+    for (int g = threadIdx.x; g < ng; g += 1024)
+        take_slot(slot, kGroupMax - (gstart[g + 1] - gstart[g]));
+    __syncthreads();
+    if (threadIdx.x < 32) {  // kGroupMax = 32 sizes
+        const int c = slot[threadIdx.x];
+        const int incl = warp_incl_scan(c);
+        __syncwarp();
+        slot[threadIdx.x] = incl - c;
+    }
+    __syncthreads();
+    for (int g = threadIdx.x; g < ng; g += 1024)
+        order[take_slot(slot, kGroupMax - (gstart[g + 1] - gstart[g]))] = g;
+}
+
 int sms_now()
 {
     int dev = 0, sms = 148;
@@ -245,7 +289,7 @@ int group_count_blocks(int n) { return (n + kChunk - 1) / kChunk > 0 ? (n + kChu
 size_t group_flag_bytes(int n) { return static_cast<size_t>(group_count_blocks(n)) * kChunk; }
 
 void launch_groups(const TreeArrays& t, int n, int gmax, int root_level,
-                   const unsigned long long* keys, GroupTable& g, cudaStream_t s)
+                   const unsigned long long* keys, GroupTable& g, bool order, cudaStream_t s)
 {
     gmax = gmax < 1 ? 1 : (gmax > kGroupMax ? kGroupMax : gmax);
     cudaMemsetAsync(g.flag, 0, group_flag_bytes(n), s);
@@ -266,6 +310,11 @@ void launch_groups(const TreeArrays& t, int n, int gmax, int root_level,
     count_launch();
     k_flag_emit<<<blocks, kThreads, 0, s>>>(g.flag, n, g.block_sums, g.ngroups, g.gstart, g.groot,
                                             keys, root_level > 0 ? g.sysroot : nullptr);
+    if (!order)
+        return;
+    // (an octree walk keeps 16 warps an SM resident)
+    count_launch();
+    k_group_order<<<1, 1024, 0, s>>>(g.gstart, g.ngroups, 16 * sms, g.order, g.ordered);
 }
 
 } // namespace bz

@@ -159,13 +159,18 @@ struct GroupTable {
     int* block_sums;  // [group_count_blocks(n)]
     int* groot;       // [n]: node where each group's walk starts (its system's root)
     int* sysroot;     // [kMaxSystems]: root node of each system (ensembles)
+    int* order;       // [kOrderGroups] groups by falling size, when *ordered
+    int* ordered;     // [1]
 };
+// Systems of up to this many groups are walked in order of falling group size.
+constexpr int kOrderGroups = 32768;
 int group_count_blocks(int n);
 size_t group_flag_bytes(int n);
 // root_level: level of the system roots (0 for one system, kSystemLevels for ensembles, whose
-// system id the sorted keys carry in bits 54..62)
+// system id the sorted keys carry in bits 54..62).  order: whether a small system's groups are
+// also ordered by size (else *g.ordered stays as it is, 0)
 void launch_groups(const TreeArrays& t, int n, int gmax, int root_level,
-                   const unsigned long long* keys, GroupTable& g, cudaStream_t s);
+                   const unsigned long long* keys, GroupTable& g, bool order, cudaStream_t s);
 
 struct WalkOutputs {
     float* ax;        // accumulated into (+=)

@@ -1099,6 +1099,8 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
                                                        TreeArrays t, const int* __restrict__ gstart,
                                                        const int* __restrict__ groot,
                                                        const int* __restrict__ ngroups_ptr,
+                                                       const int* __restrict__ gorder,
+                                                       const int* __restrict__ gordered,
                                                        WalkParams p_in, float inv_box,
                                                        WalkOutputs o, unsigned* queue,
                                                        int* spill_base, int* err)
@@ -1116,6 +1118,7 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
     WarpSmem<QUAD>& w = reinterpret_cast<WarpSmem<QUAD>*>(smem_raw)[warp];
     int* spill = spill_base + static_cast<size_t>(blockIdx.x * kWarps + warp) * kSpill;
     const int ngroups = *ngroups_ptr;
+    const bool ordered = *gordered != 0;
     if (lane == 0)
         mbar_init(&w.bar, 1);
     fence_mbar_init();
@@ -1137,6 +1140,8 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
         g = __shfl_sync(kFullMask, g, 0);
         if (g >= ngroups)
             break;
+        if (ordered)
+            g = gorder[g];
         const int g0 = gstart[g];
         const int members = gstart[g + 1] - g0;
         const float4 member = pos4[lane < members ? g0 + lane : g0];
@@ -1470,7 +1475,7 @@ void launch_variant(const float4* pos4, int n, const TreeArrays& t, const GroupT
     k_zero_u32<<<1, 1, 0, s>>>(queue);
     count_launch();
     k_walk<PERIODIC, SPLIT, QUAD, POT><<<l.blocks, kWarps * 32, l.smem, s>>>(
-        pos4, n, t, g.gstart, g.groot, g.ngroups, p, inv_box, o, queue, spill, err);
+        pos4, n, t, g.gstart, g.groot, g.ngroups, g.order, g.ordered, p, inv_box, o, queue, spill, err);
 }
 
 template <bool PERIODIC, bool SPLIT>
