@@ -49,9 +49,9 @@ struct DeviceBuffers {
     int* err = nullptr;
     double* dt = nullptr;  // {dt, dt/2}
     double* energy = nullptr;  // energy/momentum reduction scratch + results
-    unsigned* queue = nullptr;
     int* spill = nullptr;
-    unsigned long long* counters = nullptr;  // [3] listed pp, pn, evaluated pp
+    // [3] listed pp, pn, evaluated pp, then the walk's group queue: cleared together before a walk
+    unsigned long long* counters = nullptr;
     float* stage = nullptr;                  // 10n floats for host transfers
     float* ref_xyzm = nullptr;               // 4n floats, caller order, reference mode
     float4* ref_orig = nullptr;              // n float4, caller order
@@ -245,6 +245,11 @@ void enqueue_order(bz_handle* h)
     h->cur = nxt;
 }
 
+unsigned* walk_queue(const DeviceBuffers& d)
+{
+    return reinterpret_cast<unsigned*>(d.counters + 3);
+}
+
 // TreePM with the mesh leg on the second stream (outside phase timing).
 bool mesh_concurrent(const bz_handle* h)
 {
@@ -288,14 +293,9 @@ void enqueue_forces(bz_handle* h, bool kick, bool want_pot, bool mesh_forked = f
     record(h, kPhMesh);
     if (h->cfg.solver == BZ_SOLVER_TREEPM && h->pm && !overlap) {
         pm_forces(h->pm, d.pos4, n, d.acc[0], d.acc[1], d.acc[2], h->stream);
-    } else {
-        for (int a = 0; a < 3; ++a)
-            cudaMemsetAsync(d.acc[a], 0, sizeof(float) * n, h->stream);
     }
-    if (want_pot)
-        cudaMemsetAsync(d.pot, 0, sizeof(float) * n, h->stream);
     record(h, kPhWalk);
-    cudaMemsetAsync(d.counters, 0, 3 * sizeof(unsigned long long), h->stream);
+    cudaMemsetAsync(d.counters, 0, 4 * sizeof(unsigned long long), h->stream);
     WalkOutputs o{};
     o.ax = d.acc[0];
     o.ay = d.acc[1];
@@ -305,8 +305,8 @@ void enqueue_forces(bz_handle* h, bool kick, bool want_pot, bool mesh_forked = f
     WalkParams wp = walk_params(h, want_pot);
     wp.active = h->walk_active;
     wp.blocks_per_sm = h->walk_blocks_per_sm;
-    // the mesh force computed in line is already in d.acc: the walk clamps the sum
-    wp.clamp_total = h->cfg.solver == BZ_SOLVER_TREEPM && h->pm && !overlap ? 1 : 0;
+    // the mesh force computed in line is already in d.acc: the walk adds to it and clamps the sum
+    wp.add_total = h->cfg.solver == BZ_SOLVER_TREEPM && h->pm && !overlap ? 1 : 0;
     const bool learned = h->learn.enabled && h->learn.trained && h->cfg.solver == BZ_SOLVER_TREEPM;
     if (learned) {
         o.pair_src = h->learn.pair_src;
@@ -315,7 +315,7 @@ void enqueue_forces(bz_handle* h, bool kick, bool want_pot, bool mesh_forked = f
                          static_cast<float>(h->cfg.box_length / h->cfg.treepm_grid_size);
         wp.rcorr2 = std::min(rc * rc, wp.rcut2);
     }
-    launch_walk(d.pos4, n, h->tree, h->groups, wp, o, d.queue, d.spill, d.err, h->stream);
+    launch_walk(d.pos4, n, h->tree, h->groups, wp, o, walk_queue(d), d.spill, d.err, h->stream);
     // the mesh leg's accelerations complete d.acc here, or inside the closing kick
     const bool add_in_kick = overlap && kick && !learned;
     if (overlap) {
@@ -687,7 +687,7 @@ bz_status bz_create(const bz_config* cfg, size_t capacity, bz_handle** out)
     ok = ok && dalloc(h, &d.pot, n) && dalloc(h, &d.keys, n) && dalloc(h, &d.perm, n) &&
          dalloc(h, &d.box, 1) && dalloc(h, &d.bbox32, 8) && dalloc(h, &d.err, 1) &&
          dalloc(h, &d.dt, 2) && dalloc(h, &d.energy, energy_scratch_doubles()) &&
-         dalloc(h, &d.queue, 1) && dalloc(h, &d.counters, 3) &&
+         dalloc(h, &d.counters, 4) &&
          dalloc(h, &d.stage, 10 * n) && dalloc(h, &d.ref_xyzm, 4 * n) && dalloc(h, &d.ref_orig, n) &&
          dalloc(h, &d.ref_hot8, 8);
     // sort workspace
@@ -1543,10 +1543,8 @@ bz_status adaptive_steps(bz_handle* h, double dt, uint32_t nsteps)
             double* const* st = d.st[h->cur];
             launch_adaptive_active(d.id[h->cur], n, h->ad.st, sub, L, h->ad.active, h->stream);
             record(h, kPhMesh);
-            for (int a = 0; a < 3; ++a)
-                cudaMemsetAsync(d.acc[a], 0, sizeof(float) * n, h->stream);
             record(h, kPhWalk);
-            cudaMemsetAsync(d.counters, 0, 3 * sizeof(unsigned long long), h->stream);
+            cudaMemsetAsync(d.counters, 0, 4 * sizeof(unsigned long long), h->stream);
             WalkOutputs o{};
             o.ax = d.acc[0];
             o.ay = d.acc[1];
@@ -1554,7 +1552,7 @@ bz_status adaptive_steps(bz_handle* h, double dt, uint32_t nsteps)
             o.totals = d.counters;
             WalkParams wp = walk_params(h, false);
             wp.active = h->ad.active;
-            launch_walk(d.pos4, n, h->tree, h->groups, wp, o, d.queue, d.spill, d.err, h->stream);
+            launch_walk(d.pos4, n, h->tree, h->groups, wp, o, walk_queue(d), d.spill, d.err, h->stream);
             record(h, kPhIntegrate);
             launch_adaptive_close(d.acc[0], d.acc[1], d.acc[2], st[3], st[4], st[5], d.id[h->cur],
                                   h->ad.active, n, p, h->ad.st, sub, L, h->stream);

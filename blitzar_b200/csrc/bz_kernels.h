@@ -147,7 +147,7 @@ struct WalkParams {
     int blocks_per_sm;            // > 0: at most this many resident walk blocks per SM (room
                                   // for kernels of a concurrent stream); 0 = as many as fit
     float max_acc;                // acceleration clamp of the walk's sum (and of the total)
-    int clamp_total;              // the output already holds the mesh force: clamp the sum
+    int add_total;                // the output already holds the mesh force: add to it, clamp the sum
     const IsoGrid* iso;           // isolated TreePM: rsplit, rcut2, max_node_size read here
 };
 // ---------------------------------------------------------------- target groups (bz_groups.cu)

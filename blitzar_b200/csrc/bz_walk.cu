@@ -1388,19 +1388,21 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
         }
         if (valid) {
             // the walk's sum is clamped, and so is its sum with a mesh force already in the
-            // output (treePmComputeAcceleration, TpmTreeForce.inl:9-25; OctGpu.inl:227)
+            // output (treePmComputeAcceleration, TpmTreeForce.inl:9-25; OctGpu.inl:227); without one
+            // the output is only written
             float fx = acc.total(0), fy = acc.total(1), fz = acc.total(2);
             clamp_acceleration(fx, fy, fz, p.max_acc);
-            fx += o.ax[ti];
-            fy += o.ay[ti];
-            fz += o.az[ti];
-            if (p.clamp_total)
+            if (p.add_total) {
+                fx += o.ax[ti];
+                fy += o.ay[ti];
+                fz += o.az[ti];
                 clamp_acceleration(fx, fy, fz, p.max_acc);
+            }
             o.ax[ti] = fx;
             o.ay[ti] = fy;
             o.az[ti] = fz;
             if (POT && o.pot)
-                o.pot[ti] += acc.total(3);
+                o.pot[ti] = acc.total(3);
             if (o.pair_cnt) {
                 o.pair_cnt[ti] = min(npair, kPairSlots);
                 if (npair > kPairSlots)
@@ -1425,8 +1427,6 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
         __syncwarp();
     }
 }
-
-__global__ void k_zero_u32(unsigned* p) { *p = 0u; }
 
 struct WalkLaunch {
     int blocks = 0;
@@ -1471,8 +1471,6 @@ void launch_variant(const float4* pos4, int n, const TreeArrays& t, const GroupT
 {
     const WalkLaunch l = walk_shape<PERIODIC, SPLIT, QUAD, POT>(n, p.blocks_per_sm);
     const float inv_box = p.box > 0.0f ? 1.0f / p.box : 0.0f;
-    count_launch();
-    k_zero_u32<<<1, 1, 0, s>>>(queue);
     count_launch();
     k_walk<PERIODIC, SPLIT, QUAD, POT><<<l.blocks, kWarps * 32, l.smem, s>>>(
         pos4, n, t, g.gstart, g.groot, g.ngroups, g.order, g.ordered, p, inv_box, o, queue, spill, err);
