@@ -25,6 +25,8 @@
 
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 namespace bz {
 
 namespace {
@@ -34,7 +36,13 @@ constexpr int kStack = 128;       // shared-memory part of the traversal stack
 constexpr int kSpill = 8192;      // per-warp global spill area (oldest entries)
 constexpr int kList = 64;         // leaf list
 constexpr int kNodes = 128;       // accepted nodes evaluated per flush
-constexpr int kTile = 128;
+constexpr int kTile = 128;        // staged leaf particles
+// ... of a walk that only filters, where a lane sums the sources inside its own cutoff and a tile
+// takes as long as the lane with the most of them: 1.86 times the mean over 128 sources, 1.35 times
+// over 256 (256^3 walk 7.0 -> 6.45 ms).  A flush falls due early enough that most fit one tile (192
+// listed: 6.45, 256: 6.53).
+constexpr int kFilterTile = 256;
+constexpr int kFilterFlush = 192;
 constexpr int kMaskPitch = 40;  // a target's word q lies 8 banks past its word q - 1
 constexpr int kFlushParticles = 256;  // listed leaf particles that trigger a flush
 constexpr int kIndexBits = 26;
@@ -43,13 +51,14 @@ constexpr int kPerPairImage = 64;  // leaf code: periodic image chosen per pair
 
 constexpr int kNoShift = 21;       // shift code of the central image on all three axes
 
-template <bool QUAD> struct __align__(16) WarpSmem {
+template <bool QUAD, bool FILTER> struct __align__(16) WarpSmem {
+    static constexpr int kSources = FILTER ? kFilterTile : kTile;
     // a leaf flush and a node flush never overlap: they share their staging area
     union {
         struct {
-            float4 tile[kTile];
-            unsigned mask[kTile / 32][kMaskPitch];  // per-lane in-cutoff bits of the tile
-            uint4 brow[QUAD ? 1 : kTile / 2];  // cutoff filter: FP16 rows of half a tile's sources
+            float4 tile[kSources];
+            unsigned mask[kSources / 32 + 1][kMaskPitch];  // per-lane in-cutoff bits of the tile
+            uint4 brow[FILTER ? 32 : 1];  // cutoff filter: FP16 rows of 32 of the tile's sources
         };
         struct {
             // accepted nodes, two to an entry so that packed FP32 instructions take both:
@@ -58,17 +67,20 @@ template <bool QUAD> struct __align__(16) WarpSmem {
             float2 nd_tr[QUAD ? kNodes / 2 : 1];  // tr(Q) eps^2 (Newtonian) or -tr(Q) / 2 (split)
         };
     };
-    uint4 arow[QUAD ? 1 : 32];  // cutoff filter: FP16 rows of the targets
+    uint4 arow[FILTER ? 32 : 1];  // cutoff filter: FP16 rows of the targets
     float4 frame;     // ... centre of the group, scale (0: too wide for FP16, scalar filter)
     float4 tgt[32];   // the group's targets (slots past its size repeat the first)
-    int tidx[kTile];  // sorted index of each tile source (pairs recorded, potentials)
+    // sorted index of each tile source (potentials, pairs recorded); FILTER: its list entry
+    std::conditional_t<FILTER, unsigned char, int> tidx[kSources];
     unsigned stack[kStack];  // opened nodes: first child | (children - 1) << kIndexBits
     int nlist[kNodes + 32];
     int lstart[kList];
     int lcount[kList];
-    int lcode[kList];
-    int lnode[kList];
-    int lpre[kList];
+    unsigned char lcode[kList];
+    union {
+        int lnode[kList];
+        int lpre[kList];  // particles listed before the entry (once the nodes have been looked at)
+    };
     unsigned long long bar;
 };
 
@@ -484,6 +496,8 @@ template <int R, int C> struct Rows {
 // multipole_order 1), which the per-lane cutoff filter dominates: its few node terms do not pay
 // for the registers of the chunks.
 template <bool SPLIT, bool QUAD> constexpr bool walk_sliced() { return !SPLIT || QUAD; }
+// Walks whose leaves all go through the cutoff filter (in larger tiles, on the tensor cores).
+template <bool SPLIT, bool QUAD, bool POT> constexpr bool walk_filters() { return SPLIT && !QUAD && !POT; }
 
 // Calls body with every chunk of at most kChunk rows: body(std::integral_constant<R>, row0).
 template <bool SLICED, class F> __device__ __forceinline__ void for_rows(const LaneMap& lm, F body)
@@ -500,8 +514,8 @@ template <bool SLICED, class F> __device__ __forceinline__ void for_rows(const L
 }
 
 // Evaluates the first m <= kNodes listed nodes for the group's targets.
-template <bool PERIODIC, bool SPLIT, bool QUAD, bool POT>
-__device__ __forceinline__ void flush_nodes(WarpSmem<QUAD>& w, int m, const TreeArrays& t,
+template <bool PERIODIC, bool SPLIT, bool QUAD, bool POT, class W>
+__device__ __forceinline__ void flush_nodes(W& w, int m, const TreeArrays& t,
                                             const WalkParams& p, float inv2rs, const LaneMap& lm,
                                             Acc& acc)
 {
@@ -631,7 +645,7 @@ __device__ __forceinline__ void flush_nodes(WarpSmem<QUAD>& w, int m, const Tree
 }
 
 // ---- cutoff filter on the tensor cores -----------------------------------------------------
-// Which of a tile's 128 sources lie inside each of the 32 targets' cutoff spheres: the signs of
+// Which of 128 tile sources lie inside each of the 32 targets' cutoff spheres: the signs of
 //   D = |s|^2 - 2 s t + |t|^2 - r^2 = [-2t, 1, 1, Thi, Tlo] . [s, Shi, Slo, 1, 1],
 // a 32 x 128 x 8 product (mma m16n8k8, FP16 operands, FP32 sums), s and t in units of r_cut / 8
 // from the group's centre.  S = |s|^2 of the ROUNDED s and T = |t|^2 - r^2 are split into two FP16
@@ -683,8 +697,9 @@ __device__ __forceinline__ void filter_group(W& w, const float4 me, const float*
         w.frame = make_float4(gc[0], gc[1], gc[2], ext <= kFilterMaxExtent && d < kFilterScale ? sc : 0.0f);
 }
 
-// Fills w.mask for the nb sources of the tile: bit b of word q of target j is source 32 q + b.
-template <class W> __device__ __forceinline__ void filter_tile(W& w, int nb, const float4 frame)
+// Fills w.mask for the tile's sources base .. base + 127 (of nb): bit b of word q of target j is
+// source 32 q + b.
+template <class W> __device__ __forceinline__ void filter_tile(W& w, int base, int nb, const float4 frame)
 {
     const int lane = threadIdx.x & 31;
     const int row = lane >> 2, q = lane & 3;
@@ -694,57 +709,49 @@ template <class W> __device__ __forceinline__ void filter_tile(W& w, int nb, con
     for (int i = 0; i < 4; ++i)
         a[i] = ar[(row + 8 * i) * 4 + q];
     unsigned m[4] = {0u, 0u, 0u, 0u};
-    const uint32_t bbase = smem_u32(w.brow) + lane * 16;
+    // column n of n-tile t of part h is source 32 (n / 2) + 8 h + 2 t + n % 2
+    const int col = base + 32 * ((lane & 7) >> 1) + 2 * (lane >> 3) + (lane & 1);
 #pragma unroll 1
-    for (int h = 1; h >= 0; --h) {
-        // column n of n-tile t of this half is source 32 (n / 2) + 16 h + 2 t + n % 2
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int rr = lane + 32 * u, n = rr & 7;
-            const int j = 32 * (n >> 1) + 16 * h + 2 * (rr >> 3) + (n & 1);
-            uint4 v = make_uint4(0u, pack_h2(0.0f, 30000.0f), 0u, 0u);  // past the end: never inside
-            if (j < nb) {
-                const float4 s4 = w.tile[j];
-                float x = (s4.x - frame.x) * frame.w, y = (s4.y - frame.y) * frame.w, z = (s4.z - frame.z) * frame.w;
-                const float s2 = round_point(x, y, z);
-                const float hi = __half2float(__float2half_rn(s2));
-                v = make_uint4(pack_h2(x, y), pack_h2(z, hi), pack_h2(s2 - hi, 1.0f), pack_h2(1.0f, 0.0f));
-            }
-            w.brow[rr] = v;
+    for (int h = 3; h >= 0; --h) {
+        uint4 v = make_uint4(0u, pack_h2(0.0f, 30000.0f), 0u, 0u);  // past the end: never inside
+        if (col + 8 * h < nb) {
+            const float4 s4 = w.tile[col + 8 * h];
+            float x = (s4.x - frame.x) * frame.w, y = (s4.y - frame.y) * frame.w, z = (s4.z - frame.z) * frame.w;
+            const float s2 = round_point(x, y, z);
+            const float hi = __half2float(__float2half_rn(s2));
+            v = make_uint4(pack_h2(x, y), pack_h2(z, hi), pack_h2(s2 - hi, 1.0f), pack_h2(1.0f, 0.0f));
         }
+        w.brow[lane] = v;
         __syncwarp();
+        unsigned b[4];
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
+                     : "r"(smem_u32(w.brow) + lane * 16)
+                     : "memory");
 #pragma unroll
-        for (int g = 1; g >= 0; --g) {
-            unsigned b[4];
-            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3])
-                         : "r"(bbase + g * 512)
-                         : "memory");
+        for (int t = 3; t >= 0; --t) {
 #pragma unroll
-            for (int t = 3; t >= 0; --t) {
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    float c[4];
-                    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
-                        "{%7, %7, %7, %7};"
-                        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-                        : "r"(a[2 * i]), "r"(a[2 * i + 1]), "r"(b[t]), "f"(0.0f));
-                    m[2 * i] = __funnelshift_l(__float_as_uint(c[1]), m[2 * i], 1);
-                    m[2 * i] = __funnelshift_l(__float_as_uint(c[0]), m[2 * i], 1);
-                    m[2 * i + 1] = __funnelshift_l(__float_as_uint(c[3]), m[2 * i + 1], 1);
-                    m[2 * i + 1] = __funnelshift_l(__float_as_uint(c[2]), m[2 * i + 1], 1);
-                }
+            for (int i = 0; i < 2; ++i) {
+                float c[4];
+                asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+                    "{%7, %7, %7, %7};"
+                    : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                    : "r"(a[2 * i]), "r"(a[2 * i + 1]), "r"(b[t]), "f"(0.0f));
+                m[2 * i] = __funnelshift_l(__float_as_uint(c[1]), m[2 * i], 1);
+                m[2 * i] = __funnelshift_l(__float_as_uint(c[0]), m[2 * i], 1);
+                m[2 * i + 1] = __funnelshift_l(__float_as_uint(c[3]), m[2 * i + 1], 1);
+                m[2 * i + 1] = __funnelshift_l(__float_as_uint(c[2]), m[2 * i + 1], 1);
             }
         }
         __syncwarp();
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        w.mask[q][row + 8 * i] = m[i];
+        w.mask[(base >> 5) + q][row + 8 * i] = m[i];
     __syncwarp();
 }
 
-template <bool PERIODIC, bool SPLIT, bool POT, bool SLICED, class W>
+template <bool PERIODIC, bool SPLIT, bool POT, bool SLICED, bool FILTER, class W>
 __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure, const float4* __restrict__ pos4,
                                              const TreeArrays& t, const WalkParams& p,
                                              float inv2rs, bool cut, float tx, float ty, float tz,
@@ -849,8 +856,9 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
     sk.pk = 0.3275911f * inv2rs;
     sk.c2 = kTwoOverSqrtPi * inv2rs;
     int jfirst = 0;
-    for (int cbase = 0; cbase < total; cbase += kTile) {
-        const int cend = min(cbase + kTile, total);
+    constexpr int kSources = W::kSources;
+    for (int cbase = 0; cbase < total; cbase += kSources) {
+        const int cend = min(cbase + kSources, total);
         // make earlier generic-proxy reads of the tile visible before the async writes
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -873,7 +881,7 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
                 }
                 if (rec || POT)
                     for (int q = lo; q < hi; ++q)
-                        w.tidx[q - cbase] = w.lstart[first + j] + (q - w.lpre[first + j]);
+                        w.tidx[q - cbase] = FILTER ? j : w.lstart[first + j] + (q - w.lpre[first + j]);
             }
         }
         const bool any_shift = PERIODIC && __any_sync(kFullMask, shifted);
@@ -913,7 +921,7 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
             if (packed) {
                 for (int j = nb + lane; j < npad; j += 32) {
                     w.tile[j] = make_float4(tx, ty, tz, 0.0f);
-                    if (POT)
+                    if constexpr (POT)
                         w.tidx[j] = -1;
                 }
                 __syncwarp();
@@ -985,9 +993,12 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
             const float rc2n = __uint_as_float(__float_as_uint(p.rcut2) + 1u);
             // the walks that only filter mark on the tensor cores; then a marked pair takes the
             // pair law's own distance test
-            const float4 frame = SLICED ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : w.frame;
-            if (!SLICED && frame.w > 0.0f)
-                filter_tile(w, nb, frame);
+            const float4 frame = FILTER ? w.frame : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (FILTER && frame.w > 0.0f) {
+                filter_tile(w, 0, nb, frame);
+                if (nb > 128)
+                    filter_tile(w, 128, nb, frame);
+            }
             for (int wd = 0; frame.w == 0.0f && wd < nw; ++wd) {
                 const int qb = wd << 5;
                 unsigned m = 0u;
@@ -1011,19 +1022,55 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
                 }
                 w.mask[wd][lane] = m;
             }
-            int wd = 0;
-            unsigned m = w.mask[0][lane];
-            for (;;) {
-                while (m == 0u && ++wd < nw)
-                    m = w.mask[wd][lane];
-                if (m == 0u)
-                    break;
-                const int b = __ffs(m) - 1;
-                m &= m - 1u;
-                const float4 s4 = w.tile[(wd << 5) + b];
-                evald += pair_fast<SPLIT>(s4, tx, ty, tz, p.eps2, p.rcut2, !SLICED, sk, fx, fy, fz);
-                if (rec)
-                    record(s4, w.tidx[(wd << 5) + b]);
+            if constexpr (FILTER) {
+                // This lane's words with a mark, moved together, a zero word behind them; each
+                // word's place in the tile, four bits a word.  The lanes then stay in step: no lane
+                // looks for its next word while the others wait (256^3 walk 7.26 -> 7.0 ms at 128
+                // sources a tile).
+                unsigned order = 0u;
+                int used = 0;
+                for (int wd = 0; wd < nw; ++wd) {
+                    const unsigned v = w.mask[wd][lane];
+                    if (v != 0u) {
+                        w.mask[used][lane] = v;
+                        order |= static_cast<unsigned>(wd) << (4 * used);
+                        ++used;
+                    }
+                }
+                w.mask[used][lane] = 0u;
+                unsigned m = w.mask[0][lane], mnext = w.mask[1][lane];
+                int at = 1;
+                while (m != 0u) {
+                    const int b = static_cast<int>((order & 15u) << 5) + __ffs(m) - 1;
+                    m &= m - 1u;
+                    const float4 s4 = w.tile[b];
+                    const bool last = m == 0u;
+                    m = last ? mnext : m;
+                    order = last ? order >> 4 : order;
+                    at += last && mnext != 0u ? 1 : 0;
+                    mnext = w.mask[at][lane];
+                    evald += pair_fast<SPLIT>(s4, tx, ty, tz, p.eps2, p.rcut2, true, sk, fx, fy, fz);
+                    if (rec) {
+                        const int j = first + w.tidx[b];
+                        record(s4, w.lstart[j] + (cbase + b - w.lpre[j]));
+                    }
+                }
+            } else {
+                // (few leaves are filtered here: 1 % of an isolated TreePM pass is lost to the above)
+                int wd = 0;
+                unsigned m = w.mask[0][lane];
+                for (;;) {
+                    while (m == 0u && ++wd < nw)
+                        m = w.mask[wd][lane];
+                    if (m == 0u)
+                        break;
+                    const int b = (wd << 5) + __ffs(m) - 1;
+                    m &= m - 1u;
+                    const float4 s4 = w.tile[b];
+                    evald += pair_fast<SPLIT>(s4, tx, ty, tz, p.eps2, p.rcut2, false, sk, fx, fy, fz);
+                    if (rec)
+                        record(s4, w.tidx[b]);
+                }
             }
             __syncwarp();
             // (jfirst, the first leaf the unfiltered path below must look at, is left behind
@@ -1082,13 +1129,14 @@ __device__ __forceinline__ void flush_leaves(W& w, int first, int nl, bool sure,
     }
 }
 
-// Resident blocks an SM that the walk is compiled for (4: 128 registers, 5: 96, 7: 72).  The
+// Resident blocks an SM that the walk is compiled for (4: 128 registers, 5: 96, 6: 80).  The
 // sliced evaluation keeps two nodes, two targets and their sums in packed registers: 4 blocks
 // hold them without spills (Hernquist 4M: 36.4 ms at 4, 37.4 at 5; isolated TreePM 1M: 4.35 at 4,
-// 4.45 at 5, 4.99 at 6).  The walk that only filters takes the warps.
+// 4.45 at 5, 4.99 at 6).  The walk that only filters takes the warps that its tile leaves room for
+// (6 blocks, 80 registers: 256^3 6.45 ms, 5: 6.81).
 template <bool SPLIT, bool QUAD, bool POT> constexpr int walk_min_blocks()
 {
-    return SPLIT && !QUAD && !POT ? 7 : 4;
+    return walk_filters<SPLIT, QUAD, POT>() ? 6 : 4;
 }
 
 // Persistent kernel: each warp takes groups from a global queue until none are left.  The
@@ -1115,7 +1163,9 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
     }
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    WarpSmem<QUAD>& w = reinterpret_cast<WarpSmem<QUAD>*>(smem_raw)[warp];
+    constexpr bool FILTER = walk_filters<SPLIT, QUAD, POT>();
+    using Smem = WarpSmem<QUAD, FILTER>;
+    Smem& w = reinterpret_cast<Smem*>(smem_raw)[warp];
     int* spill = spill_base + static_cast<size_t>(blockIdx.x * kWarps + warp) * kSpill;
     const int ngroups = *ngroups_ptr;
     const bool ordered = *gordered != 0;
@@ -1183,7 +1233,7 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
             ghalf[a] = __fmul_rn(0.5f, __fsub_rn(gmax[a], gmin[a]));
         }
 
-        if (!SLICED && cut)
+        if (FILTER && cut)
             filter_group(w, me, gc, ghalf, rcut);
         // With a cutoff, leaves wholly inside it for every target ("sure": the farthest corners of
         // leaf and group) are listed from the far end of the leaf list and summed without the
@@ -1372,12 +1422,12 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
                     w.nlist[lane] = e;
                 __syncwarp();
             }
-            if (nl + ns >= (done ? 1 : 32) || lp >= kFlushParticles) {
+            if (nl + ns >= (done ? 1 : 32) || lp >= (FILTER ? kFilterFlush : kFlushParticles)) {
 #pragma unroll 1
                 for (int part = 0; part < (SLICED ? 2 : 1); ++part) {
                     const int cnt = part ? ns : nl;
                     if (cnt > 0)
-                        flush_leaves<PERIODIC, SPLIT, POT, SLICED>(
+                        flush_leaves<PERIODIC, SPLIT, POT, SLICED, FILTER>(
                             w, part ? kList - ns : 0, cnt, part != 0, pos4, t, p, inv2rs, cut, me.x, me.y,
                             me.z, ti, acc, phase, err, o, valid ? ti : -1, npair, evald, lanes);
                 }
@@ -1444,7 +1494,7 @@ WalkLaunch walk_shape(int n, int blocks_per_sm)
     WalkLaunch local;
     WalkLaunch& c = (dev >= 0 && dev < kMaxDevices) ? cached[dev] : local;
     if (c.blocks == 0) {
-        const size_t smem = sizeof(WarpSmem<QUAD>) * kWarps;
+        const size_t smem = sizeof(WarpSmem<QUAD, walk_filters<SPLIT, QUAD, POT>()>) * kWarps;
         cudaFuncSetAttribute(k_walk<PERIODIC, SPLIT, QUAD, POT>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         int sms = 148, per_sm = 1;
