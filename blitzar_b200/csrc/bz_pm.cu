@@ -608,18 +608,16 @@ __global__ void __launch_bounds__(kThreads) k_apply_green(cufftComplex* __restri
     }
 }
 
-// Fused Green x spectral gradient: F_a = i k_a G rho_k for a = x, y, z (Nyquist derivative
-// terms set to zero).
 // ---- z transform, Green's function and inverse z transform in one pass ------------------------
 // After the 2-D transforms of the planes, each column of M coefficients along z is transformed,
 // multiplied by the Green's function and transformed back without leaving the SM: one read and
-// one write of the spectrum and one read of the table (1.35 GB at 512^3) where a 3-D plan pair and a separate
-// multiplication move it three times.  HBM and shared memory: 512^3 0.40 ms (3.4 TB/s) where the two
-// z passes and the multiplication took 0.88 ms; 128^3, in the L2, 7.2 us against 17.
+// one write of the spectrum and one read of the table where a 3-D plan pair and a separate
+// multiplication move it three times.  Bound by the L2 and shared memory: 7.2 us at 128^3 where the
+// two z passes and the multiplication took 17.
 //
 // A block takes kZCols neighbouring columns (128-byte rows), eight points a thread.  The transform is
 // decimated in frequency, M = 8 x 8 x M/64: radix 8 over z = j + r M/8, radix 8 within each
-// residue, a last radix M/64; the inverse runs the same steps backwards, so that every exchange
+// residue, a last radix 2 when M = 128; the inverse runs the same steps backwards, so that every exchange
 // writes the places it read and the frequencies need no reordering.
 constexpr int kZCols = 16;
 
@@ -637,7 +635,7 @@ template <bool INV> __device__ __forceinline__ float2 crot(float2 a)
     return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
-template <bool INV> __device__ __forceinline__ void radix2(float2& a, float2& b)
+__device__ __forceinline__ void radix2(float2& a, float2& b)
 {
     const float2 t = a;
     a = cadd(t, b);
@@ -670,19 +668,12 @@ template <bool INV> __device__ __forceinline__ void radix8(float2* x)
     x[6] = csub(e2, o2);
     x[7] = csub(e3, o3);
 }
-// Transforms of L consecutive points each, in place.
-template <int L, bool INV> __device__ __forceinline__ void radix_last(float2* x)
+// The last transforms, of two neighbouring points each.
+__device__ __forceinline__ void radix_last(float2* x)
 {
-    if constexpr (L == 8) {
-        radix8<INV>(x);
-    } else if constexpr (L == 4) {
-        radix4<INV>(x[0], x[1], x[2], x[3]);
-        radix4<INV>(x[4], x[5], x[6], x[7]);
-    } else if constexpr (L == 2) {
 #pragma unroll
-        for (int g = 0; g < 8; g += 2)
-            radix2<INV>(x[g], x[g + 1]);
-    }
+    for (int g = 0; g < 8; g += 2)
+        radix2(x[g], x[g + 1]);
 }
 
 template <int M>
@@ -723,7 +714,7 @@ __global__ void __launch_bounds__(kZCols * M / 8) k_z_green(float2* __restrict__
 #pragma unroll
         for (int r = 0; r < 8; ++r)
             x[r] = own[r * kZCols];
-        radix_last<M2, false>(x);
+        radix_last(x);
     }
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
@@ -735,7 +726,7 @@ __global__ void __launch_bounds__(kZCols * M / 8) k_z_green(float2* __restrict__
         x[r].y *= g;
     }
     if constexpr (M2 > 1) {
-        radix_last<M2, true>(x);
+        radix_last(x);
 #pragma unroll
         for (int r = 0; r < 8; ++r)
             own[r * kZCols] = x[r];
@@ -765,10 +756,14 @@ __global__ void __launch_bounds__(kZCols * M / 8) k_z_green(float2* __restrict__
             spec[(j + r * M1) * plane + col] = x[r];
 }
 
-// Mesh sides k_z_green is built for: powers of two whose eight points a thread and kZCols columns
-// make a block of at most 1024 threads and whose last radix is at most 8.  Other sides (the
-// isolated mesh's 2 G, 32 and below, 1024 and above) keep the 3-D transforms.
-bool z_fused_side(int m) { return m == 64 || m == 128 || m == 256 || m == 512; }
+// Mesh sides k_z_green serves.  Its potential and that of cuFFT's 3-D transforms carry FP32 rounding
+// of the same size, but not the same rounding, and differentiation divides it by the cell: the mesh
+// forces of the two differ by about 1.3e-8 of the force times the side (measured 0.6e-6 at 64, 1.6e-6
+// at 128, 3.3e-6 at 256, 6.3e-6 at 512).  Forces of this path are held to 5e-6 from one version to the
+// next, which leaves no margin at 256 and is passed at 512: those sides keep the 3-D transforms (512^3:
+// 0.88 against 0.40 ms for the z passes and the multiplication), as do the isolated mesh's 2 G and
+// sides of 32 and below.
+bool z_fused_side(int m) { return m == 64 || m == 128; }
 
 template <int M> cudaError_t z_green_launch(const PmPlan* p, cudaStream_t s)
 {
@@ -797,8 +792,6 @@ int z_green(const PmPlan* p, cudaStream_t s)
     switch (p->mesh) {
     case 64: e = z_green_launch<64>(p, s); break;
     case 128: e = z_green_launch<128>(p, s); break;
-    case 256: e = z_green_launch<256>(p, s); break;
-    case 512: e = z_green_launch<512>(p, s); break;
     default: break;
     }
     return e == cudaSuccess ? 0 : 3;
@@ -813,6 +806,8 @@ __global__ void k_twiddles(int m, float2* tw)
     }
 }
 
+// Fused Green x spectral gradient: F_a = i k_a G rho_k for a = x, y, z (Nyquist derivative
+// terms set to zero).
 __global__ void __launch_bounds__(kThreads) k_green_gradient(const cufftComplex* __restrict__ spec,
                                                               const float* __restrict__ green,
                                                               int mesh, double box,

@@ -1,6 +1,7 @@
-"""The periodic mesh solve at every side the fused z transform is built for and one on each side of
-them, against the same Green's function applied in FP64; and the tensor-core cutoff filter's pair
-counts against the FP64 distances."""
+"""The periodic mesh solve at the sides with the fused z transform and at those on each side of them,
+against the same Green's function applied in FP64, by the potential and by its forces; the large sides
+against cuFFT's 3-D FP32 transforms; and the tensor-core cutoff filter's pair counts against the FP64
+distances."""
 import numpy as np
 import pytest
 
@@ -30,6 +31,70 @@ def test_potential_matches_fp64_solve(gpu, mesh, gradient, assign):
     ref = np.fft.irfftn(np.fft.rfftn(rho) * green, s=rho.shape, axes=(0, 1, 2))
     # two FP32 transforms of M^3 points: a few 2^-24 sqrt(log2 M^3) of the norm, far below 2e-6
     assert np.linalg.norm(phi - ref) < 2e-6 * np.linalg.norm(ref)
+
+
+def _lattice_solve(mesh, gradient, assign):
+    """Density and potential meshes of a displaced lattice of half the side, and the Green's function
+    of the solve in FP64, on the GPU.  2^k particles of mass 2^-k at eighths of a cell: the sums of a CIC
+    deposit are exact, so it repeats whatever the order of its atomics."""
+    import torch
+
+    from blitzar_b200 import ics
+    from blitzar_b200._lib import Engine
+
+    rs = 0.95
+    pos, _, m = ics.grf_grid(mesh // 2, seed=mesh)
+    pos = np.rint(pos * (8 * mesh)) / (8 * mesh) % 1.0
+    with Engine(len(m), solver=1, box_length=1.0, treepm_grid_size=mesh, treepm_r_split_cells=rs,
+                treepm_assignment=assign, treepm_gradient=gradient, treepm_window_floor=0.08) as e:
+        e.set_state(pos, None, m.astype(np.float32), f64=True)
+        rho, phi = (torch.from_numpy(e.pm_mesh(w)).cuda().reshape(1, mesh, mesh, mesh) for w in (0, 1))
+    k = 2 * np.pi * torch.fft.fftfreq(mesh, 1 / mesh, dtype=torch.float64, device="cuda")
+    kr = 2 * np.pi * torch.fft.rfftfreq(mesh, 1 / mesh, dtype=torch.float64, device="cuda")
+    k2 = k[:, None, None] ** 2 + k[None, :, None] ** 2 + kr[None, None, :] ** 2
+    s, sr = torch.sinc(k / (2 * np.pi * mesh)), torch.sinc(kr / (2 * np.pi * mesh))
+    window = (s[:, None, None] * s[None, :, None] * sr[None, None, :]) ** (2 * (assign + 2))
+    k2[0, 0, 0] = 1.0
+    green = 4 * np.pi * torch.exp(-k2 * (rs / mesh) ** 2) / (k2 * window.clamp_min(0.08))
+    green[0, 0, 0] = 0.0
+    return rho, phi, green
+
+
+def _force_difference(a, b):
+    """2-norm of the difference of two potentials' centred differences over that of b's."""
+    num = den = 0.0
+    for axis in (1, 2, 3):
+        d = [(f.roll(-1, axis) - f.roll(1, axis)).double() for f in (a.double(), b.double())]
+        num += float(((d[0] - d[1]) ** 2).sum())
+        den += float((d[1] ** 2).sum())
+    return (num / den) ** 0.5
+
+
+@pytest.mark.parametrize("mesh", [64, 128, 256, 512])
+@pytest.mark.parametrize("gradient,assign", [(0, 0), (2, 2)])
+def test_mesh_forces_match_fp64_solve(gpu, mesh, gradient, assign):
+    """The potential's FP32 rounding, a few 2^-24 of its norm, which the longest waves fill, divided by
+    the cell: of the order of 2^-24 (6e-8) / pi of the force times the side, whatever the transforms."""
+    import torch
+
+    rho, phi, green = _lattice_solve(mesh, gradient, assign)
+    ref = torch.fft.irfftn(torch.fft.rfftn(rho.double(), dim=(1, 2, 3)) * green, s=(mesh,) * 3, dim=(1, 2, 3))
+    assert _force_difference(phi, ref) < 2 * 2.0 ** -24 / np.pi * mesh
+
+
+@pytest.mark.parametrize("mesh", [256, 512])
+@pytest.mark.parametrize("gradient", [0, 2])
+def test_large_sides_round_as_the_3d_transforms(gpu, mesh, gradient):
+    """Sides of 256 and more give cuFFT's 3-D FP32 solve, rounding included.  torch's (the batch axis
+    has it plan all three axes at once) shares the forward rounding bit for bit; a table entry an FP32
+    unit away redraws part of the inverse's: 0.4 to 0.6e-8 of the force times the side.  A solve by
+    other transforms lies 1.5 to 1.7e-8 away."""
+    import torch
+
+    rho, phi, green = _lattice_solve(mesh, gradient, 0)
+    spec = torch.fft.rfftn(rho, dim=(1, 2, 3)) * green.float()
+    ref = torch.fft.irfftn(spec, s=(mesh,) * 3, dim=(1, 2, 3))
+    assert _force_difference(phi, ref) < 1e-8 * mesh
 
 
 def _pairs_box(side, shift, seed):
