@@ -154,6 +154,7 @@ template <class T> bool dalloc(bz_handle* h, T** p, size_t count)
     void* q = nullptr;
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
     if (cudaMalloc(&q, bytes) != cudaSuccess) {
+        cudaGetLastError();  // reported by the caller: a later call is not to find it
         *p = nullptr;
         return false;
     }
@@ -161,6 +162,12 @@ template <class T> bool dalloc(bz_handle* h, T** p, size_t count)
     h->bytes += bytes;
     *p = static_cast<T*>(q);
     return true;
+}
+
+// An array made at its first use: a call that ran out of memory part-way leaves the rest to the next.
+template <class T> bool dalloc_once(bz_handle* h, T** p, size_t count)
+{
+    return *p || dalloc(h, p, count);
 }
 
 bool periodic(const bz_handle* h) { return h->cfg.solver == BZ_SOLVER_TREEPM && h->cfg.box_length > 0.0; }
@@ -1823,20 +1830,16 @@ namespace {
 bool learn_alloc(bz_handle* h)
 {
     auto& L = h->learn;
-    if (L.params)
-        return true;
-    return dalloc(h, &L.params, kMlpParams) && dalloc(h, &L.grad, kMlpParams) &&
-           dalloc(h, &L.adam_m, kMlpParams) && dalloc(h, &L.adam_v, kMlpParams) &&
-           dalloc(h, &L.loss, 1);
+    return dalloc_once(h, &L.params, kMlpParams) && dalloc_once(h, &L.grad, kMlpParams) &&
+           dalloc_once(h, &L.adam_m, kMlpParams) && dalloc_once(h, &L.adam_v, kMlpParams) &&
+           dalloc_once(h, &L.loss, 1);
 }
 
 bool learn_pairs_alloc(bz_handle* h)
 {
     auto& L = h->learn;
-    if (L.pair_src)
-        return true;
-    return dalloc(h, &L.pair_src, h->capacity * static_cast<size_t>(kPairSlots)) &&
-           dalloc(h, &L.pair_cnt, h->capacity) && dalloc(h, &L.feat, h->capacity);
+    return dalloc_once(h, &L.pair_src, h->capacity * static_cast<size_t>(kPairSlots)) &&
+           dalloc_once(h, &L.pair_cnt, h->capacity) && dalloc_once(h, &L.feat, h->capacity);
 }
 
 void drop_graphs(bz_handle* h)
