@@ -54,6 +54,23 @@ def test_mlp_forward_matches_oracle(gpu, oracle):
     assert np.median(err) < 2e-3 and err.max() < 3e-2, (np.median(err), err.max())
 
 
+@pytest.mark.parametrize("depth", [-30.0, -41.4, -41.6, -90.0, -1e3, -1e20, -1e30])
+def test_mlp_deep_negative_activations_vanish(gpu, oracle, depth):
+    """Pre-activations around and far below the value at which the two-at-a-time activation stops:
+    SiLU goes to 0 there (its own minimum is -0.28), next to ordinary ones in the same row."""
+    p = _params(6)
+    p[15:512:32] = depth  # b1 of every other unit
+    p[1536:1568:3] = depth  # b2 of every third
+    x = _inputs(300, 7)
+    with _engine() as e:
+        e.learn_set(p, 1.0)
+        y = e.learn_forward(x).astype(np.float64)
+    ref = oracle.mlp_forward(p, x, 1.0).astype(np.float64)
+    err = np.linalg.norm(y - ref, axis=1) / np.maximum(np.linalg.norm(ref, axis=1), 1e-3)
+    # as test_mlp_forward_matches_oracle
+    assert np.median(err) < 2e-3 and err.max() < 3e-2, (np.median(err), err.max())
+
+
 def test_mlp_gradient_matches_oracle(gpu, oracle):
     p = _params(3)
     x = _inputs(512, 4)
