@@ -231,10 +231,10 @@ __global__ void __launch_bounds__(kThreads) k_flag_emit(const unsigned char* __r
         gstart[*ngroups] = n;
 }
 
-// slot[s]++, one atomic for the lanes of a warp that share s.
-__device__ __forceinline__ int take_slot(int* slot, int s)
+// slot[s]++, one atomic for the lanes of `lanes` (those that call) that share s.
+__device__ __forceinline__ int take_slot(unsigned lanes, int* slot, int s)
 {
-    const unsigned peers = __match_any_sync(__activemask(), s);
+    const unsigned peers = __match_any_sync(lanes, s);
     const int leader = __ffs(peers) - 1;
     int at = 0;
     if ((threadIdx.x & 31) == leader)
@@ -261,8 +261,13 @@ __global__ void __launch_bounds__(1024) k_group_order(const int* __restrict__ gs
     if (threadIdx.x < kGroupMax)
         slot[threadIdx.x] = 0;
     __syncthreads();
-    for (int g = threadIdx.x; g < ng; g += 1024)
-        take_slot(slot, kGroupMax - (gstart[g + 1] - gstart[g]));
+    // (whole warps stay in the loops: the lanes that take a slot are named by a vote before they do)
+    for (int g0 = threadIdx.x & ~31; g0 < ng; g0 += 1024) {
+        const int g = g0 + (threadIdx.x & 31);
+        const unsigned lanes = __ballot_sync(kFullMask, g < ng);
+        if (g < ng)
+            take_slot(lanes, slot, kGroupMax - (gstart[g + 1] - gstart[g]));
+    }
     __syncthreads();
     if (threadIdx.x < 32) {  // kGroupMax = 32 sizes
         const int c = slot[threadIdx.x];
@@ -271,8 +276,12 @@ __global__ void __launch_bounds__(1024) k_group_order(const int* __restrict__ gs
         slot[threadIdx.x] = incl - c;
     }
     __syncthreads();
-    for (int g = threadIdx.x; g < ng; g += 1024)
-        order[take_slot(slot, kGroupMax - (gstart[g + 1] - gstart[g]))] = g;
+    for (int g0 = threadIdx.x & ~31; g0 < ng; g0 += 1024) {
+        const int g = g0 + (threadIdx.x & 31);
+        const unsigned lanes = __ballot_sync(kFullMask, g < ng);
+        if (g < ng)
+            order[take_slot(lanes, slot, kGroupMax - (gstart[g + 1] - gstart[g]))] = g;
+    }
 }
 
 int sms_now()
