@@ -1459,19 +1459,18 @@ __global__ void __launch_bounds__(kWarps * 32, walk_min_blocks<SPLIT, QUAD, POT>
                     raise_error(err, kErrListCapacity);
             }
         }
-        unsigned long long ev = __reduce_add_sync(kFullMask, valid ? evald : 0u);
-        if (adaptive)  // (the counters report the walked groups' members)
-            ev = static_cast<unsigned long long>(cnt_pp) * members;
+        const unsigned ev = __reduce_add_sync(kFullMask, valid ? evald : 0u);
         if (lane == 0) {
             if (o.n_pp)
                 o.n_pp[g] = cnt_pp;
             if (o.n_pn)
                 o.n_pn[g] = cnt_pn;
             if (o.totals) {
-                const unsigned long long ng = static_cast<unsigned long long>(members);
+                // (of the targets evaluated: in adaptive substeps not the whole group)
+                const unsigned long long ng = static_cast<unsigned long long>(gn);
                 atomicAdd(&o.totals[0], ng * cnt_pp);
                 atomicAdd(&o.totals[1], ng * cnt_pn);
-                atomicAdd(&o.totals[2], ev);
+                atomicAdd(&o.totals[2], static_cast<unsigned long long>(ev));
             }
         }
         __syncwarp();

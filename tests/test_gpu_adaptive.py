@@ -60,3 +60,23 @@ def test_adaptive_energy_conservation(gpu):
         lv = e.adaptive_levels()
     assert lv.max() >= 2  # the run did use several levels
     assert abs((k1 + w1) - (k0 + w0)) < 1e-3 * abs(k0 + w0)
+
+
+@pytest.mark.parametrize("eta", [1e6, 0.02])
+def test_counters_count_the_targets_evaluated(gpu, eta):
+    """A block's last substep closes every particle, so its counters are a whole walk's: with one
+    level (a fresh tree) those of a plain evaluation of the same positions; without a cutoff every
+    listed pair is taken through the pair law."""
+    from blitzar_b200 import ics
+
+    n = 20_000
+    pos, vel, m = ics.plummer(n, seed=9)
+    with _engine(n, octree_theta=0.5, octree_softening=0.01, adaptive_max_level=5, adaptive_eta=eta) as e:
+        e.set_state(pos, vel, m.astype(np.float32), f64=True)
+        e.step(4e-3, 1)
+        block = e.walk_counts()
+        e.accelerations()
+        plain = e.walk_counts()
+    assert block[0] == block[1] and plain[0] == plain[1]
+    if eta > 1:
+        assert block == plain
