@@ -112,7 +112,6 @@ struct bz_handle {
         int* lmax = nullptr;
         bool ready = false;               // levels and cached accelerations match the state
     } ad;
-    const unsigned char* walk_active = nullptr;  // mask handed to the walk (adaptive substeps)
     // ensembles of independent systems (0 = one system)
     int systems = 0;
     long long* sys_offsets = nullptr;  // [kMaxSystems + 1] caller-index offsets
@@ -310,7 +309,6 @@ void enqueue_forces(bz_handle* h, bool kick, bool want_pot, bool mesh_forked = f
     o.pot = want_pot ? d.pot : nullptr;
     o.totals = d.counters;
     WalkParams wp = walk_params(h, want_pot);
-    wp.active = h->walk_active;
     wp.blocks_per_sm = h->walk_blocks_per_sm;
     // the mesh force computed in line is already in d.acc: the walk adds to it and clamps the sum
     wp.add_total = h->cfg.solver == BZ_SOLVER_TREEPM && h->pm && !overlap ? 1 : 0;

@@ -143,7 +143,9 @@ struct WalkParams {
     int quadrupole;
     int want_pot;
     float rcorr2;     // > 0 with WalkOutputs.pair_src: record the pairs closer than this
-    const unsigned char* active;  // optional [n]: walk only groups with an active target
+    // optional [n], for adaptive substeps: only targets whose flag is set are evaluated and written.
+    // Octree force walks only: with a box, a split or potentials it is not read (no caller sets it there).
+    const unsigned char* active;
     int blocks_per_sm;            // > 0: at most this many resident walk blocks per SM (room
                                   // for kernels of a concurrent stream); 0 = as many as fit
     float max_acc;                // acceleration clamp of the walk's sum (and of the total)
