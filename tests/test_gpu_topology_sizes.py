@@ -37,6 +37,24 @@ def test_topology_and_order_match_oracle(gpu, oracle, n, leaf):
         assert np.array_equal(t[name], o[name]), name
 
 
+@pytest.mark.parametrize("n", [600_001, (1 << 20) - 1, (1 << 20) + 1, (1 << 23) - 1, (1 << 23) + 4097])
+def test_topology_of_large_systems(gpu, oracle, n):
+    """2, 4 and 16 particles a thread, and scans of more than 1024 block counts."""
+    pos = plummer(n, seed=n)
+    pos[:: n // 40] = pos[0]
+    m = np.full(n, 1.0 / n, np.float32)
+    p64 = pos.astype(np.float64)
+    lo = p64.min(0)
+    keys = oracle.morton63(p64, lo, float((p64.max(0) - lo).max()))
+    perm = oracle.stable_sort(keys)
+    o = oracle.build_tree(keys[perm], oracle.pos4(pos[perm], m[perm]), leaf_cap=16)
+    t, k, p = _tree(n, pos, m, leaf_capacity=16)
+    assert np.array_equal(k, keys[perm]) and np.array_equal(p, perm)
+    assert t["nodes"] == o["nodes"]
+    for name in ("start", "count", "child", "nchild", "mono", "bmin", "bmax", "quad"):
+        assert np.array_equal(t[name], o[name]), name
+
+
 def test_node_capacity_overflow_is_reported(gpu):
     """Close pairs far apart need a chain of single-child nodes each: more nodes than the arrays
     hold.  The build stops at the last level that fits and reports the limit."""
