@@ -80,3 +80,64 @@ def test_counters_count_the_targets_evaluated(gpu, eta):
     assert block[0] == block[1] and plain[0] == plain[1]
     if eta > 1:
         assert block == plain
+
+
+def _direct(pos, mass, eps):
+    d = pos[None] - pos[:, None]
+    return ((mass[None] * ((d * d).sum(-1) + eps * eps) ** -1.5)[..., None] * d).sum(1)
+
+
+def _level(a, v, eta, eps, dt, top):
+    am, vm = np.linalg.norm(a, axis=1), np.linalg.norm(v, axis=1)
+    stable = np.minimum(dt, np.minimum(eta * np.sqrt(eps / np.maximum(am, 1e-6)), eta * eps / np.maximum(vm, 1e-6)))
+    return np.minimum(np.ceil(np.log2(dt / stable) - 1e-9).astype(int).clip(0), top)
+
+
+def _block(pos, vel, mass, eps, dt, eta, top):
+    """One block of hierarchical kick-drift-kick steps in FP64 with direct sums; returns the state and how
+    often each particle closed a step."""
+    acc = _direct(pos, mass, eps)
+    level = _level(acc, vel, eta, eps, dt, top)
+    L = int(level.max())
+    closed = np.zeros(len(pos), int)
+    for s in range(1 << L):
+        opens = s % (1 << (L - level)) == 0
+        vel = vel + np.where(opens[:, None], 0.5 * dt / (1 << level)[:, None] * acc, 0.0)
+        pos = pos + dt / (1 << L) * vel
+        closes = (s + 1) % (1 << (L - level)) == 0
+        fresh = _direct(pos, mass, eps)
+        acc = np.where(closes[:, None], fresh, acc)
+        vel = vel + np.where(closes[:, None], 0.5 * dt / (1 << level)[:, None] * acc, 0.0)
+        last = s + 1 == 1 << L
+        coarsest = 0 if last else L - ((s + 1) & -(s + 1)).bit_length() + 1
+        want = np.clip(_level(acc, vel, eta, eps, dt, top), coarsest, top if last else L)
+        level = np.where(closes, want, level)
+        closed += closes
+    return pos, vel, closed
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("gsize", [1, 2, 5, 32])
+def test_substeps_move_every_particle_as_direct_sums_do(gpu, order, gsize):
+    """Substeps evaluate the closing members of a group, from one to all of them: with the opening angle
+    near zero the block is that of FP64 direct sums, particle by particle, and closes as many steps."""
+    from blitzar_b200 import ics
+
+    n, eps, dt, eta, top = 900, 0.02, 8e-3, 0.05, 6
+    pos, vel, m = ics.plummer(n, seed=21)
+    mass = m.astype(np.float32)
+    p, v, closed = _block(pos, vel, mass.astype(np.float64), eps, dt, eta, top)
+    assert len(np.unique(closed)) >= 4  # several levels
+    with _engine(n, octree_theta=1e-3, physics_min_theta=1e-3, octree_softening=eps, multipole_order=order,
+                 walk_group_size=gsize, adaptive_max_level=top, adaptive_eta=eta) as e:
+        e.set_state(pos, vel, mass, f64=True)
+        e.step(dt, 1)
+        gp, gv = e.get_state(f64=True)
+        updates = e.adaptive_updates()
+    kick = dt * np.linalg.norm(_direct(pos, mass.astype(np.float64), eps), axis=1)
+    err = np.linalg.norm(gv - v, axis=1) / kick
+    # FP32 sums of n terms; a particle whose level falls on the other side of the rule's comparison (none
+    # of these seeds) would take other steps, one that was given another's force would be off by order 1
+    assert err.max() < 1e-4, (err.max(), np.argmax(err))
+    assert np.abs(gp - p).max() < 1e-4 * dt * kick.max()
+    assert updates == closed.sum()
