@@ -49,8 +49,17 @@ struct SortWorkspace {
     unsigned long long* state;   // [max_tiles][256] look-back words
     int max_tiles;
 };
-size_t sort_state_words(int n);
-int sort_tile_items();
+// Keys a tile holds, and the size below which the tiles are short.
+constexpr int kSortTileLong = 4096, kSortTileShort = 2048, kSortShortKeys = 1 << 19;
+// Look-back words: the most tiles of any n' <= n (a workspace serves every smaller sort).
+constexpr size_t sort_state_words(int n)
+{
+    const int few = n < kSortShortKeys ? 0 : (n + kSortTileLong - 1) / kSortTileLong;
+    const int small = n < kSortShortKeys ? n : kSortShortKeys - 1;
+    const int many = (small + kSortTileShort - 1) / kSortTileShort;
+    const int t = few > many ? few : many;
+    return static_cast<size_t>(t < 1 ? 1 : t) * 256;
+}
 // Stable LSD radix sort of (keys, vals) on the low `bits` key bits (multiple of 8).  The
 // sorted result lands back in (keys, vals).
 void launch_radix_sort(unsigned long long* keys, uint32_t* vals, int n, int bits,
@@ -175,10 +184,10 @@ void launch_groups(const TreeArrays& t, int n, int gmax, int root_level,
                    const unsigned long long* keys, GroupTable& g, bool order, cudaStream_t s);
 
 struct WalkOutputs {
-    float* ax;        // accumulated into (+=)
+    float* ax;        // written (with WalkParams.add_total: added to what is there)
     float* ay;
     float* az;
-    float* pot;       // optional (+=)
+    float* pot;       // optional
     unsigned long long* n_pp;  // optional per-group counters
     unsigned long long* n_pn;
     unsigned long long* totals; // optional [3]: listed pairs, node terms (x targets), pairs

@@ -27,8 +27,7 @@ constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
 constexpr size_t kMaxKeys = BZ_SORT_NOALLOC_MAX_KEYS;
-constexpr size_t kTileItems = 2048;  // onesweep tile; checked against sort_tile_items()
-constexpr size_t kStateWords = (kMaxKeys + kTileItems - 1) / kTileItems * 256;
+constexpr size_t kStateWords = bz::sort_state_words(static_cast<int>(kMaxKeys));
 
 constexpr size_t kOffKeys = 0;
 constexpr size_t kOffVals = align_up(kOffKeys + 8 * kMaxKeys);
@@ -39,7 +38,7 @@ constexpr size_t kOffTicket = align_up(kOffBase + 4 * 8 * 256);
 constexpr size_t kOffEpoch = align_up(kOffTicket + 4 * 8);
 constexpr size_t kOffTrivial = align_up(kOffEpoch + 4);
 constexpr size_t kOffErr = align_up(kOffTrivial + 4 * 8);
-constexpr size_t kScratchBytes = align_up(kOffErr + 4);  // 13.1 MiB for 2^20 keys
+constexpr size_t kScratchBytes = align_up(kOffErr + 4);  // 12.6 MiB for 2^20 keys
 
 // The scratch.  In host code this name is only a host-side stand-in for the symbol: the
 // device address comes from cudaGetSymbolAddress, once per device (scratch_on_device).
@@ -93,9 +92,6 @@ extern "C" bz_status bz_sort_pairs_noalloc(uint64_t* keys, uint32_t* values, int
     if (reinterpret_cast<uintptr_t>(keys) % alignof(uint64_t) != 0 ||
         reinterpret_cast<uintptr_t>(values) % alignof(uint32_t) != 0)
         return BZ_INVALID_ARGUMENT;
-    if (static_cast<size_t>(bz::sort_tile_items()) != kTileItems ||
-        bz::sort_state_words(static_cast<int>(n)) > kStateWords)
-        return BZ_INTERNAL_ERROR;
 
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= bz::kMaxDevices)

@@ -1,6 +1,6 @@
 // Stable LSD radix sort of (u64 key, u32 value) pairs: one histogram pass over the keys for
 // all digit positions, then one single-pass ("onesweep") kernel per 8-bit digit that ranks a
-// 4096-key tile in shared memory, obtains its global digit offsets through decoupled
+// tile of 4096 keys (2048 below 2^19) in shared memory, obtains its global digit offsets through decoupled
 // look-back, and scatters.  Replaces thrust::sort_by_key in
 // engine/physics/octree/cuda/linear/OctBuild.inl:96 (CUB radix sort, stable), with which it
 // agrees bit for bit (same stable order).
@@ -16,14 +16,13 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-// Keys per lane and tile.  Below kShortTileKeys keys the tiles are half as long: a pass is then the
+// Keys per lane and tile.  Below kSortShortKeys keys the tiles are half as long: a pass is then the
 // time of the one tile an SM takes, not of the memory (whole sorts of 60 thousand pairs 149 ->
 // 130 us, of 300 thousand 170 -> 156 us; of a million no difference); above, long tiles halve the
 // look-back words.
-constexpr int kIterLong = 16, kIterShort = 8;
-constexpr int kShortTileKeys = 1 << 19;
-constexpr int tile_keys(int iter) { return kWarps * 32 * iter; }
-int sort_iter(int n) { return n < kShortTileKeys ? kIterShort : kIterLong; }
+constexpr int kIterLong = kSortTileLong / kThreads, kIterShort = kSortTileShort / kThreads;
+constexpr int tile_keys(int iter) { return kThreads * iter; }
+int sort_iter(int n) { return n < kSortShortKeys ? kIterShort : kIterLong; }
 // Predecessors a look-back step reads at once.  The tiles of a pass start together, so late ones
 // look back over many of them; one at a time, that chain of loads was 1.5 of the 22 us of a pass
 // of a million keys.
@@ -301,17 +300,6 @@ __global__ void k_fixup(unsigned long long* keys_a, uint32_t* vals_a,
 }
 
 } // namespace
-
-int sort_tile_items() { return tile_keys(kIterShort); }
-
-size_t sort_state_words(int n)
-{
-    // the most tiles of any n' <= n: a workspace serves every smaller sort
-    auto tiles = [](int m) { return (m + tile_keys(sort_iter(m)) - 1) / tile_keys(sort_iter(m)); };
-    const int few = tiles(n), many = tiles(n < kShortTileKeys ? n : kShortTileKeys - 1);
-    const int t = few > many ? few : many;
-    return static_cast<size_t>(t < 1 ? 1 : t) * 256;
-}
 
 namespace {
 

@@ -339,7 +339,7 @@ bz_status bz_learn_gradient(bz_handle* h, const float* x6, const float* y3, int6
  * accounting), and step loops where cudaMalloc/cudaFree are too costly (cudaFree waits for
  * the whole device).  The handle-based API above allocates in bz_create; this call does
  * not: its scratch is a fixed array in device memory, sized for BZ_SORT_NOALLOC_MAX_KEYS
- * pairs (about 13.1 MiB), that every process loading this library holds on each device it
+ * pairs (about 12.6 MiB), that every process loading this library holds on each device it
  * uses until exit.  It calls no cudaMalloc, cudaFree or allocating library routine.
  *
  * keys/values: device (or managed) memory of the current device, n entries each; sorted by

@@ -1,4 +1,4 @@
-"""The all-levels-at-once topology and the one-block sort at the sizes where they can go wrong:
+"""The all-levels-at-once topology and the small sort by counting at the sizes where they can go wrong:
 around block and run sizes, leaf capacities from one particle to more than the system holds,
 duplicates down to the depth limit, and a node count past the array's capacity."""
 import numpy as np
