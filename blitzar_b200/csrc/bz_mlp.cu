@@ -55,14 +55,13 @@ struct __align__(1024) MlpSmem {
     __nv_bfloat16 w3t[kHid * kOutPad];   // B  W3^T (columns 3..15 zero) LBO 128 SBO 256
     float b2[kHid];
     float b3[4];
-    float red[2][3];
     unsigned long long bar;
     uint32_t tmem;
 };
 
 // Inference needs only the forward operands: one hidden buffer serves both layers (H2 is
 // written after the second product has consumed H1), and tensor memory holds D1 / D3 in
-// columns 0.. and D2 in 32.. (D3 is written after D1 has been read out).  17 KB of shared
+// columns 0.. and D2 in 32.. (D3 is written after D1 has been read out).  17 to 20 KB of shared
 // memory and 64 TMEM columns a block, so eight blocks share an SM (512 columns).
 constexpr uint32_t kInferCols = 64;
 constexpr uint32_t kInferD1 = 0, kInferD2 = 32, kInferD3 = 0;
@@ -76,7 +75,6 @@ struct __align__(1024) MlpInferSmem {
     __nv_bfloat16 w3[kOutPad * kHid];    // B  W3 (rows 3..15 zero)
     float b2[kHid];
     float b3[4];
-    float red[2][3];
     unsigned long long bar;
     uint32_t tmem;
 };
@@ -684,7 +682,7 @@ __global__ void k_adam(float* __restrict__ p, float* __restrict__ g, float* __re
 }
 
 size_t mlp_smem() { return sizeof(MlpSmem) + 1024; }
-// Inference blocks request at least 1/7 of an SM's shared memory so that no more than
+// Inference blocks request more than a ninth of an SM's shared memory so that no more than
 // kInferBlocksPerSm of them (whose TMEM columns add up to the SM's 512) are ever co-resident:
 // a ninth block's tcgen05.alloc would otherwise wait for a column range to be freed.
 size_t mlp_infer_smem()
