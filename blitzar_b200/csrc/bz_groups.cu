@@ -242,6 +242,14 @@ __device__ __forceinline__ int take_slot(unsigned lanes, int* slot, int s)
     return __shfl_sync(peers, at, leader) + __popc(peers & lanemask_lt());
 }
 
+// Place of a group among the sizes, the largest first.  (Groups hold 1 to kGroupMax particles; after a
+// sort that gave up, whose error the call reports, the cuts may lie anywhere: bounded, so that no slot
+// outside the array is touched.)
+__device__ __forceinline__ int size_rank(const int* __restrict__ gstart, int g)
+{
+    return kGroupMax - max(1, min(gstart[g + 1] - gstart[g], kGroupMax));
+}
+
 // The order in which the walk takes the groups of a small system: by falling size (a counting sort
 // over the sizes in one block; equal sizes in any order, which no result depends on).  A walk of a
 // few groups a warp ends when its last long group does, so the long ones go first (Plummer 65k,
@@ -266,7 +274,7 @@ __global__ void __launch_bounds__(1024) k_group_order(const int* __restrict__ gs
         const int g = g0 + (threadIdx.x & 31);
         const unsigned lanes = __ballot_sync(kFullMask, g < ng);
         if (g < ng)
-            take_slot(lanes, slot, kGroupMax - (gstart[g + 1] - gstart[g]));
+            take_slot(lanes, slot, size_rank(gstart, g));
     }
     __syncthreads();
     if (threadIdx.x < 32) {  // kGroupMax = 32 sizes
@@ -280,7 +288,7 @@ __global__ void __launch_bounds__(1024) k_group_order(const int* __restrict__ gs
         const int g = g0 + (threadIdx.x & 31);
         const unsigned lanes = __ballot_sync(kFullMask, g < ng);
         if (g < ng)
-            order[take_slot(lanes, slot, kGroupMax - (gstart[g + 1] - gstart[g]))] = g;
+            order[take_slot(lanes, slot, size_rank(gstart, g))] = g;
     }
 }
 
