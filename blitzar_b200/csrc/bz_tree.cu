@@ -38,7 +38,7 @@ constexpr int kLevels = kMaxLevels + 1;  // levels 0 .. kMaxLevels
 // each level, and an emission.  A kernel a level (binary searches for the octant boundaries of
 // every node, a look-back scan) chained 21 launches of 1 to 38 us.  Topology time, level chain ->
 // this: Plummer 65k 163 -> 22 us, isolated TreePM 1M 390 -> 83 us, Hernquist 4M 680 -> 135 us,
-// the 256^3 lattice 298 -> 314 us (the tree phase with it 0.73 -> 0.67 ms).  Bound by latency below a
+// the 256^3 lattice 319 -> 243 us (the tree phase with it 0.73 -> 0.62 ms).  Bound by latency below a
 // million particles (four launches), by the issue of the key comparisons above.
 
 // Octant digits two keys share (0 .. kMaxLevels).
@@ -262,12 +262,11 @@ __global__ void __launch_bounds__(kThreads) k_tree_emit(const unsigned long long
                 t.parent[k] = above;
                 t.level[k] = l;
                 t.arrive[k] = 0;
+                t.nchild[k] = 0;
                 if (l > b)
                     t.child[above] = k;  // the chain's node above starts at this particle too
-                if (l == e) {
+                if (l == e)
                     t.child[k] = -1;
-                    t.nchild[k] = 0;
-                }
             }
             above = in ? k : k - 1;
             next += lane == l ? __popc(m) : 0;
@@ -275,13 +274,16 @@ __global__ void __launch_bounds__(kThreads) k_tree_emit(const unsigned long long
     }
 }
 
-// The child count of every split node, from the last of its (consecutive) children.
+// The child count of every split node, from the last of its (consecutive) children.  Sorted keys give
+// every node but the root a split parent one level up.  After a sort that gave up (the call reports it)
+// they need not: a node without such a parent is left out of the tree, so that every link that the moments
+// and the walk follow is a node's own.
 __global__ void __launch_bounds__(kThreads) k_tree_children(TreeArrays t)
 {
     const int nn = t.n_nodes[0];
     for (int k = blockIdx.x * kThreads + threadIdx.x + 1; k < nn; k += gridDim.x * kThreads) {
         const int p = t.parent[k];
-        if (k + 1 == nn || t.parent[k + 1] != p)
+        if ((k + 1 == nn || t.parent[k + 1] != p) && p >= 0 && t.child[p] >= 0 && t.level[p] + 1 == t.level[k])
             t.nchild[p] = k - t.child[p] + 1;
     }
 }
